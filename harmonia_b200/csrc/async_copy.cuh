@@ -70,6 +70,19 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, int x, 
       : "memory");
 }
 
+// Asynchronous copy of one 4- or 8-byte element to shared memory (this
+// thread's copies are waited for together).
+template <typename T>
+__device__ __forceinline__ void cp_async_element(T *dst, const T *src) {
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "4 or 8 bytes");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(sizeof(T)) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Orders this thread's earlier generic-proxy accesses to shared memory
 // before later async-proxy (TMA) writes to it.
 __device__ __forceinline__ void fence_proxy_async_smem() {

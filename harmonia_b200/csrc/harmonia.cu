@@ -4,7 +4,7 @@
 // drivers this replaces exit on any CUDA error
 // (CUDA_ERROR_HANDLER, open-harmonia/src/cuda_utils.h:3-12); every path here
 // returns an HM_E* code instead.
-#include "hm_internal.cuh"
+#include "bucket_sort.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -334,6 +334,17 @@ bool is_device_ptr(const void *p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Device memory that this device's kernels can read as int64 in place.
+bool readable_here(const void *p, int dev) {
+  cudaPointerAttributes a;
+  if (((uintptr_t)p & 7) != 0) return false;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
 bool is_pinned_host(const void *p) {
   if (!p) return false;
   cudaPointerAttributes a;
@@ -647,7 +658,10 @@ int hm_bulk_load(const int64_t *keys, const int64_t *vals, size_t n_, const hm_c
   // Temporaries: two key and two value buffers for the sort, sort scratch, flags.
   int64_t tn = std::max<int64_t>(std::max<int64_t>(n, t->n_leaf), 1);
   size_t tb = align_up(tn * 8, 256);
-  size_t temp_bytes = 4 * tb + align_up((int64_t)radix_scratch_bytes(n), 256) + 256;
+  const bool bucketed = bsort::fits(n);
+  size_t sort_bytes = radix_scratch_bytes(n);
+  if (bucketed) sort_bytes = std::max(sort_bytes, bsort::work_bytes(n));
+  size_t temp_bytes = 4 * tb + align_up((int64_t)sort_bytes, 256) + 256;
   char *temp = nullptr;
   e = dev_alloc(&t->arena, total);
   if (e == cudaSuccess) e = dev_alloc(reinterpret_cast<void **>(&temp), temp_bytes);
@@ -672,19 +686,64 @@ int hm_bulk_load(const int64_t *keys, const int64_t *vals, size_t n_, const hm_c
   void *sort_scratch = temp + 4 * tb;
   unsigned *flags = reinterpret_cast<unsigned *>(temp + temp_bytes - 256);
   cudaStream_t s = 0;
-  cudaMemsetAsync(t->arena, 0, total, s);
   cudaMemsetAsync(t->d_err, 0, 256, s);
-  cudaMemsetAsync(flags, 0, 4, s);
-  if (n > 0) {
-    // keys land in uk_alt as int64, are sign-flipped into uk, values go to vv
-    e = cudaMemcpyAsync(uk_alt, keys, n * 8, cudaMemcpyDefault, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(vv, vals, n * 8, cudaMemcpyDefault, s);
+  const int64_t *in_k = keys, *in_v = vals;
+  if (n > 0) {  // what the kernels cannot read where it lies is copied
+    e = cudaSuccess;
+    if (!readable_here(keys, dev)) {
+      e = cudaMemcpyAsync(uk, keys, n * 8, cudaMemcpyDefault, s);
+      in_k = reinterpret_cast<const int64_t *>(uk);
+    }
+    if (e == cudaSuccess && !readable_here(vals, dev)) {
+      e = cudaMemcpyAsync(vv, vals, n * 8, cudaMemcpyDefault, s);
+      in_v = vv;
+    }
     if (e != cudaSuccess) {
       release_after(temp, s);
       free_tree(t);
       return cuda_err(e);
     }
-    transform_keys_in(reinterpret_cast<int64_t *>(uk_alt), uk, n, s);
+  }
+  if (bucketed) {
+    bsort::Ctl *ctl = nullptr, h{};
+    rc = build_from_pairs(t->target(), in_k, in_v, n, reinterpret_cast<int64_t *>(uk_alt), vv_alt,
+                          reinterpret_cast<int64_t *>(uk), vv, sort_scratch, t->num_sms, &ctl, s);
+    if (rc == HM_OK) {
+      e = cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+      rc = cuda_err(e);
+    }
+    if (rc == HM_OK && !h.skew && h.flags) rc = (h.flags & 2u) ? HM_EMAXKEY : HM_EDUPLICATE;
+    if (rc || !h.skew) {
+      release_after(temp, s);
+      if (rc) {
+        free_tree(t);
+        return rc;
+      }
+      t->key_min = h.ends[0];
+      t->key_max = h.ends[1];
+      choose_smem_levels(t);
+      *out = t;
+      return HM_OK;
+    }
+  }
+  // no keys, more of them than the bucket sort takes, or keys that crowd one
+  // of its buckets: LSD sort, then leaves and inner levels from the sorted keys
+  cudaMemsetAsync(flags, 0, 4, s);
+  if (n > 0) {
+    // keys are sign-flipped into uk, values go to vv
+    e = cudaSuccess;
+    if (in_k != keys) {
+      e = cudaMemcpyAsync(uk_alt, in_k, n * 8, cudaMemcpyDefault, s);
+      in_k = reinterpret_cast<const int64_t *>(uk_alt);
+    }
+    if (e == cudaSuccess && in_v != vv) e = cudaMemcpyAsync(vv, in_v, n * 8, cudaMemcpyDefault, s);
+    if (e != cudaSuccess) {
+      release_after(temp, s);
+      free_tree(t);
+      return cuda_err(e);
+    }
+    transform_keys_in(in_k, uk, n, s);
     bool alt = radix_sort_pairs<int64_t>(uk, vv, uk_alt, vv_alt, n, 0, 64, sort_scratch, s);
     if (alt) {
       std::swap(uk, uk_alt);
