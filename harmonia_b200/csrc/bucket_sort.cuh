@@ -76,7 +76,8 @@ struct Ctl {
   unsigned skew;                  // a bucket over kCap: nothing is sorted
   unsigned flags;                 // bit 0: a key twice, bit 1: a key equals Max_Key
   unsigned pad;
-  int64_t ends[2];                // lowest and highest key (written by the bulk loader)
+  int64_t ends[2];                // lowest and highest key (written by the caller's last step)
+  unsigned long long user[4];     // the caller's own results
   Map map;
 };
 

@@ -1122,13 +1122,12 @@ int hm_delete_batch(hm_tree *t, const int64_t *keys, size_t n_, size_t *removed,
   }
   int64_t gone = 0;
   int tok = prof_begin(t, s);
-  int rc = delete_epoch(t, dk, n, &gone, s);
+  unsigned err = 0;
+  int rc = delete_epoch(t, dk, n, &gone, &err, s);
   prof_end(t, kStageDelete, tok, s);
-  cudaError_t e = cudaStreamSynchronize(s);
-  if (rc == HM_OK && e != cudaSuccess) rc = cuda_err(e);
   if (removed) *removed = (size_t)gone;
   choose_smem_levels(t);
-  return rc ? rc : hm_sync(t, hs);
+  return rc || !err ? rc : hm_sync(t, hs);
 }
 
 int hm_upsert_batch(hm_tree *t, const int64_t *keys, const int64_t *vals, size_t n_, int flags,
@@ -1153,12 +1152,11 @@ int hm_upsert_batch(hm_tree *t, const int64_t *keys, const int64_t *vals, size_t
     dv = tv;
   }
   int tok = prof_begin(t, s);
-  int rc = upsert_epoch(t, dk, dv, n, flags, s);
+  unsigned err = 0;
+  int rc = upsert_epoch(t, dk, dv, n, flags, &err, s);
   prof_end(t, kStageUpsert, tok, s);
-  cudaError_t e = cudaStreamSynchronize(s);
-  if (rc == HM_OK && e != cudaSuccess) rc = cuda_err(e);
   choose_smem_levels(t);
-  return rc ? rc : hm_sync(t, hs);
+  return rc || !err ? rc : hm_sync(t, hs);
 }
 
 int hm_autotune(hm_tree *t, const int64_t *sample_q, size_t n_, hm_config *best) {

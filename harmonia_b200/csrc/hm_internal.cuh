@@ -372,6 +372,8 @@ size_t scan_scratch_bytes(int64_t n);
 void exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, void *scratch,
                         cudaStream_t s);  // out has n+1 entries
 void exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, void *scratch, cudaStream_t s);
+// leaf_base = exclusive scan of leaf_cnt, unless *go (device memory) is 0.
+void rescan_leaf_base(const hm_tree *t, const unsigned long long *go, void *scratch, cudaStream_t s);
 void export_contents(const hm_tree *t, int64_t *d_keys, int64_t *d_vals, cudaStream_t s);
 size_t range_scratch_bytes(int64_t n);
 // Counts per query: the first len[i] records >= start[i] (end == nullptr), or
@@ -382,10 +384,11 @@ int range_copy_out(const hm_tree *t, const int32_t *first_leaf, const int32_t *f
                    const int64_t *offsets, int64_t n, int64_t *okeys, int64_t *ovals, cudaStream_t s);
 
 // ---- upsert (upsert.cu) ----
-int delete_epoch(hm_tree *t, const int64_t *d_keys, int64_t n, int64_t *removed, cudaStream_t s);
+// Both return when done; *err: the tree's error word during the epoch.
+int delete_epoch(hm_tree *t, const int64_t *d_keys, int64_t n, int64_t *removed, unsigned *err, cudaStream_t s);
 int rebuild_from_sorted(hm_tree *t, const uint64_t *ck, const int64_t *cv, int64_t n1, cudaStream_t s);
 int upsert_epoch(hm_tree *t, const int64_t *d_keys, const int64_t *d_vals, int64_t n,
-                 int flags, cudaStream_t s);
+                 int flags, unsigned *err, cudaStream_t s);
 
 // ---- stage timing ----
 enum Stage { kStagePartition = 0, kStageSearch, kStageBatches, kStageRange, kStageUpsert, kStageJoin,

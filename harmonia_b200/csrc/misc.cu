@@ -31,8 +31,10 @@ constexpr int kScanStep = kThreads * kScanPer;  // elements per CTA per scan ste
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) seg_sum_kernel(const T *__restrict__ in, int64_t n,
-                                                           int64_t seg, int64_t *__restrict__ part) {
+                                                           int64_t seg, int64_t *__restrict__ part,
+                                                           const unsigned long long *go) {
   pdl_enter();
+  if (go && *go == 0) return;
   __shared__ int64_t red[kThreads / 32];
   int64_t b0 = (int64_t)blockIdx.x * seg, b1 = min(n, b0 + seg);
   int64_t s = 0;
@@ -57,15 +59,18 @@ __global__ void __launch_bounds__(kThreads) seg_sum_kernel(const T *__restrict__
 }
 
 // Exclusive scan of each segment, offset by the sum of the segments before it
-// (each CTA adds up those of the at most 592 segment sums itself).  A step
+// (each CTA adds up those of the at most 592 segment sums itself); the sum of
+// all goes to *total (may be null).  go != null: nothing unless *go != 0.  A step
 // stages kScanStep elements in shared memory (coalesced), each thread scans
 // kScanPer consecutive ones (index i at i + i / 8: one pad word per 8 keeps
 // the threads' runs in different banks), one block scan of the thread sums.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) seg_scan_kernel(const T *__restrict__ in, int64_t n,
                                                             int64_t seg, const int64_t *__restrict__ part,
-                                                            int64_t *__restrict__ out, int nctas) {
+                                                            int64_t *__restrict__ out, int nctas,
+                                                            int64_t *total, const unsigned long long *go) {
   pdl_enter();
+  if (go && *go == 0) return;
   __shared__ int64_t buf[kScanStep + kScanStep / 8];
   __shared__ int64_t wsum[kThreads / 32];
   __shared__ int64_t carry;
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(kThreads) seg_scan_kernel(const T *__restrict_
     }
     __syncthreads();
   }
-  if (blockIdx.x == nctas - 1 && tid == 0) out[n] = carry;
+  if (total && blockIdx.x == nctas - 1 && tid == 0) *total = carry;
 }
 
 __global__ void export_kernel(DevTree t, int lc, int li, int64_t *__restrict__ keys,
@@ -272,8 +277,9 @@ void exclusive_scan(const T *in, int64_t *out, int64_t n, void *scratch, cudaStr
     cudaMemsetAsync(out, 0, sizeof(int64_t), s);
     return;
   }
-  launch_pdl(seg_sum_kernel<T>, nctas, kThreads, 0, s, in, n, seg, part);
-  launch_pdl(seg_scan_kernel<T>, nctas, kThreads, 0, s, in, n, seg, part, out, nctas);
+  const unsigned long long *go = nullptr;
+  launch_pdl(seg_sum_kernel<T>, nctas, kThreads, 0, s, in, n, seg, part, go);
+  launch_pdl(seg_scan_kernel<T>, nctas, kThreads, 0, s, in, n, seg, part, out, nctas, out + n, go);
   note_launch(2);
 }
 
@@ -284,6 +290,16 @@ void exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, void *scratc
 
 void exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, void *scratch, cudaStream_t s) {
   exclusive_scan<int32_t>(in, out, n, scratch, s);
+}
+
+void rescan_leaf_base(const hm_tree *t, const unsigned long long *go, void *scratch, cudaStream_t s) {
+  const int nctas = scan_ctas(t->n_leaf);
+  const int64_t seg = (t->n_leaf + nctas - 1) / nctas;
+  int64_t *part = static_cast<int64_t *>(scratch), *total = nullptr;
+  launch_pdl(seg_sum_kernel<int32_t>, nctas, kThreads, 0, s, t->leaf_cnt, t->n_leaf, seg, part, go);
+  launch_pdl(seg_scan_kernel<int32_t>, nctas, kThreads, 0, s, t->leaf_cnt, t->n_leaf, seg, part, t->leaf_base, nctas,
+             total, go);
+  note_launch(2);
 }
 
 void export_contents(const hm_tree *t, int64_t *d_keys, int64_t *d_vals, cudaStream_t s) {

@@ -585,8 +585,10 @@ void run_epoch(hm_server *sv, std::vector<Req *> &ups) {
     cudaError_t e = cudaMemcpyAsync(dk, hk, n * 8, cudaMemcpyHostToDevice, sl.s);
     if (e == cudaSuccess && !del) e = cudaMemcpyAsync(dv, hv, n * 8, cudaMemcpyHostToDevice, sl.s);
     rc = cuda_err(e);
+    unsigned err = 0;  // a search that gave up has reported to its own requests
     if (rc == HM_OK)
-      rc = del ? delete_epoch(t, dk, n, nullptr, sl.s) : upsert_epoch(t, dk, dv, n, ups[0]->r.flags, sl.s);
+      rc = del ? delete_epoch(t, dk, n, nullptr, &err, sl.s)
+               : upsert_epoch(t, dk, dv, n, ups[0]->r.flags, &err, sl.s);
     e = cudaStreamSynchronize(sl.s);
     if (rc == HM_OK) rc = cuda_err(e);
     refresh_smem_levels(t);

@@ -9,34 +9,32 @@
 // (rebuild_without_leaf, open-harmonia/src/bpt-ppi-update.cpp:320-463).  The
 // reference never refreshes the GPU copy.
 //
-// Here the epoch runs on the device tree itself (an epoch of at most 1024
-// keys whose new keys all fit their leaves in one CTA, see small_epoch_kernel;
-// otherwise in these steps):
-//   1. sort the batch by key (stable, payload = input index) and keep the
-//      last occurrence of each key;
-//   2. one thread per key descends; a hit overwrites the value in place
-//      (supplied value, or key-1 under HM_UPSERT_REF_KEY_MINUS_1);
-//   3. the misses, still in key order, are grouped by leaf; if every touched
-//      leaf has room, one warp per leaf merges its new keys into the sorted
-//      row (separators stay valid: a key routed to leaf j lies in
+// Here the epoch runs on the device tree itself, enqueued as one chain of
+// kernels whose outcome the host reads once:
+//   1. bucket sort of the batch by key (payload = input position, so the last
+//      of equal keys is known; an LSD sort where its keys crowd a bucket);
+//   2. every key descends; a hit overwrites the value in place (supplied
+//      value, or key-1 under HM_UPSERT_REF_KEY_MINUS_1), a miss sets a bit;
+//   3. the misses of one leaf are placed in its sorted row if it has room
+//      (separators stay valid: a key routed to leaf j lies in
 //      [separator_j, separator_j+1)), and leaf_base is rescanned;
-//   4. otherwise the tree is rebuilt: the current contents and the misses
-//      are merged (each element's output slot = own rank + rank in the other
-//      run) and bulk-loaded into a fresh arena with the same parameters.
-#include "hm_internal.cuh"
+//   4. if a leaf had no room, its subtree is rebalanced, or the tree is
+//      rebuilt: the current contents and the left-over keys are merged (each
+//      element's output slot = own rank + rank in the other run) and
+//      bulk-loaded into a fresh arena with the same parameters.
+#include "bucket_sort.cuh"
 
 #include <algorithm>
 #include <cstring>
 
 namespace hm {
 
-void scan_counts(int64_t *counts, int64_t m, cudaStream_t s);
-void exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, void *scratch, cudaStream_t s);
-void export_contents(const hm_tree *t, int64_t *d_keys, int64_t *d_vals, cudaStream_t s);
 
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kApply = 128;      // threads of apply_kernel
+constexpr int kRowThreads = 128;  // threads of leaf_rows_kernel
 
 unsigned grid_for(int64_t items) {
   int64_t b = (items + kThreads - 1) / kThreads;
@@ -45,346 +43,546 @@ unsigned grid_for(int64_t items) {
   return (unsigned)b;
 }
 
-// keep[i] = 1 for the last occurrence of each key in the sorted batch;
-// flags bit1 if a key equals Max_Key.
-__global__ void last_occurrence_kernel(const uint64_t *__restrict__ uk, int64_t n,
-                                       int32_t *__restrict__ keep, unsigned *flags) {
-  unsigned f = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    keep[i] = (i == n - 1 || uk[i] != uk[i + 1]) ? 1 : 0;
-    if ((int64_t)(uk[i] ^ kSign) == kMaxKey) f |= 2u;
-  }
-  if (f) atomicOr(flags, f);
+// ---- the batch in key order ----
+
+// Last step of the batch's bucket sort: a CTA sorts one bucket in shared memory
+// and writes its keys and their input positions, equal keys in input order.
+// start == nullptr: the whole batch is one bucket.
+__global__ void __launch_bounds__(bsort::kSortThreads, 5) epoch_sort_kernel(
+    const int64_t *__restrict__ keys, const int32_t *__restrict__ pos, const uint32_t *__restrict__ start, uint32_t n,
+    int64_t *__restrict__ sk, int32_t *__restrict__ spos, bsort::Ctl *ctl) {
+  pdl_enter();
+  extern __shared__ __align__(16) unsigned char dyn[];
+  auto &sm = *reinterpret_cast<bsort::SortSmem<int32_t> *>(dyn);
+  if (ctl->skew) return;
+  const uint32_t s0 = start ? start[blockIdx.x] : 0;
+  const int m = (int)((start ? start[blockIdx.x + 1] : n) - s0);
+  if (m == 0) return;
+  const bsort::Map map = ctl->map;
+  auto emit = [&](int i, int64_t k, int32_t p, bool) {
+    sk[s0 + i] = k;
+    spos[s0 + i] = p;
+    if (i == 0 || i == m - 1) {
+      if (k == kMaxKey) atomicOr(&ctl->flags, 2u);  // sorts last
+      if (s0 + i == 0) ctl->ends[0] = k;
+      if (s0 + i == n - 1) ctl->ends[1] = k;
+    }
+  };
+  if (start)
+    bsort::sort_bucket<int32_t, false>(sm, map, keys + s0, pos + s0, m, emit);
+  else
+    bsort::sort_bucket<int32_t, true>(sm, map, keys, nullptr, m, emit);
 }
 
-__global__ void compact_batch_kernel(const uint64_t *__restrict__ uk, const int32_t *__restrict__ idx,
-                                     const int64_t *__restrict__ vals, const int32_t *__restrict__ keep,
-                                     const int64_t *__restrict__ at, int64_t n,
-                                     int64_t *__restrict__ bk, int64_t *__restrict__ bv) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    if (keep[i]) {
-      int64_t o = at[i];
-      bk[o] = (int64_t)(uk[i] ^ kSign);
-      bv[o] = vals[idx[i]];
+// The same results from an LSD-sorted batch.
+__global__ void lsd_finish_kernel(const uint64_t *__restrict__ uk, int64_t n, int64_t *__restrict__ sk,
+                                  bsort::Ctl *ctl) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = (int64_t)(uk[i] ^ kSign);
+    sk[i] = k;
+    if (i == 0) ctl->ends[0] = k;
+    if (i == n - 1) {
+      ctl->ends[1] = k;
+      if (k == kMaxKey) ctl->flags = 2u;
     }
   }
 }
 
-// Small batches (the serving loop's epochs) skip the multi-pass radix sort:
-// Keys in one upsert or delete epoch, at most: the batch sort carries each
-// key's input position as an int32 (such a batch would need about 200 GB of
-// scratch anyway).
-constexpr int64_t kMaxEpochKeys = 0x7fffffff;
+// Ctl::user of an epoch.
+enum { kUserChanged = 0, kUserOverflow = 1, kUserEmpty = 2, kUserErr = 3 };  // keys added or removed; ...; error word
 
-// one CTA sorts (key, input index) pairs in shared memory with a bitonic
-// network, keeps each key's last occurrence and writes the kept keys (and
-// values) in key order to bk/bv and their number to *count; flags bit1 if a
-// key equals Max_Key.
-constexpr int kSmallSort = 2048;
+// Keys <= q in a node of 64 sorted keys of which lane l holds 2l and 2l + 1.
+__device__ __forceinline__ int warp_rank(longlong2 p, int64_t q) {
+  int pos = 0;  // lanes whose first key is <= q
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1)
+    if (__shfl_sync(0xffffffffu, p.x, pos + step - 1) <= q) pos += step;
+  if (__shfl_sync(0xffffffffu, p.x, pos) <= q) pos++;  // pos <= 31 here
+  const int64_t y = __shfl_sync(0xffffffffu, p.y, max(pos - 1, 0));
+  return pos == 0 ? 0 : 2 * pos - 1 + (y <= q);
+}
 
-__global__ void __launch_bounds__(1024) small_sort_unique_kernel(const int64_t *__restrict__ keys,
-                                                                 const int64_t *__restrict__ vals, int n,
-                                                                 int64_t *__restrict__ bk, int64_t *__restrict__ bv,
-                                                                 int64_t *__restrict__ count, unsigned *flags) {
-  __shared__ uint64_t sk[kSmallSort];
-  __shared__ int32_t si[kSmallSort];
-  __shared__ int32_t wsum[32];
-  const int tid = threadIdx.x;
-  int P = 1;
-  while (P < n) P <<= 1;
-  unsigned f = 0;
-  for (int i = tid; i < P; i += blockDim.x) {
-    const bool real = i < n;
-    const int64_t k = real ? keys[i] : 0;
-    if (real && k == kMaxKey) f |= 2u;
-    sk[i] = real ? (uint64_t)k ^ kSign : ~0ull;  // padding sorts after every real key
-    si[i] = real ? i : INT32_MAX;
+// Leaf of each of a warp's 32 keys, which are in key order.  While the lowest
+// and the highest key go to the same child the warp descends as one, with one
+// dependent load a level: a lane holds two of the node's keys, and ballots
+// count those <= a key.  Where they part, every lane ranks its key among the
+// keys the warp holds.  Below that two neighbouring nodes are still searched
+// that way; only keys that spread further search alone (two loads a level).
+__device__ __forceinline__ int32_t descend_leaf_warp(const DevTree &t, int f, int64_t q) {
+  const int ix = f / 8, row = ix + f, lane = threadIdx.x & 31;
+  const int64_t q0 = __shfl_sync(0xffffffffu, q, 0), q1 = __shfl_sync(0xffffffffu, q, 31);
+  int32_t node = 0;  // the warp's, then the lane's
+  int l = 0;
+  for (; l < t.height; l++) {
+    const int64_t *r = t.inner + (int64_t)node * row + ix;
+    const int32_t first = __ldg(t.prefix + node);
+    const longlong2 p = __ldg(reinterpret_cast<const longlong2 *>(r + 2 * lane));
+    longlong2 p2 = make_longlong2(kMaxKey, kMaxKey);
+    if (f > 64) p2 = __ldg(reinterpret_cast<const longlong2 *>(r + 64 + 2 * lane));
+    int c0 = __popc(__ballot_sync(0xffffffffu, p.x <= q0)) + __popc(__ballot_sync(0xffffffffu, p.y <= q0));
+    int c1 = __popc(__ballot_sync(0xffffffffu, p.x <= q1)) + __popc(__ballot_sync(0xffffffffu, p.y <= q1));
+    if (f > 64) {
+      c0 += __popc(__ballot_sync(0xffffffffu, p2.x <= q0)) + __popc(__ballot_sync(0xffffffffu, p2.y <= q0));
+      c1 += __popc(__ballot_sync(0xffffffffu, p2.x <= q1)) + __popc(__ballot_sync(0xffffffffu, p2.y <= q1));
+    }
+    if (c0 == c1) {
+      node = first + c0;
+      continue;
+    }
+    node = first + warp_rank(p, q);
+    if (f > 64) node += warp_rank(p2, q);
+    l++;
+    break;
   }
-  if (f) atomicOr(flags, f);
-  __syncthreads();
-  for (int k = 2; k <= P; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = tid; i < P; i += blockDim.x) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const bool asc = (i & k) == 0;
-          const bool gt = sk[i] > sk[ixj] || (sk[i] == sk[ixj] && si[i] > si[ixj]);
-          if (gt == asc) {
-            const uint64_t tk = sk[i];
-            sk[i] = sk[ixj];
-            sk[ixj] = tk;
-            const int32_t ti = si[i];
-            si[i] = si[ixj];
-            si[ixj] = ti;
-          }
-        }
+  for (; l < t.height; l++) {
+    const int32_t n0 = __shfl_sync(0xffffffffu, node, 0), n1 = __shfl_sync(0xffffffffu, node, 31);
+    if (n1 - n0 <= 1) {
+      const int64_t *ra = t.inner + (int64_t)n0 * row + ix, *rb = t.inner + (int64_t)n1 * row + ix;
+      const longlong2 pa = __ldg(reinterpret_cast<const longlong2 *>(ra + 2 * lane));
+      const longlong2 pb = __ldg(reinterpret_cast<const longlong2 *>(rb + 2 * lane));
+      const int32_t first = __ldg(t.prefix + node);
+      const int ca = warp_rank(pa, q), cb = warp_rank(pb, q);
+      int c = node == n0 ? ca : cb;
+      if (f > 64) {
+        const longlong2 pa2 = __ldg(reinterpret_cast<const longlong2 *>(ra + 64 + 2 * lane));
+        const longlong2 pb2 = __ldg(reinterpret_cast<const longlong2 *>(rb + 64 + 2 * lane));
+        const int ca2 = warp_rank(pa2, q), cb2 = warp_rank(pb2, q);
+        c += node == n0 ? ca2 : cb2;
       }
-      __syncthreads();
+      node = first + c;
+      continue;
     }
-  }
-  // keep the last occurrence of each key; two elements per thread, block scan
-  int kept[2], mine = 0;
-  for (int h = 0; h < 2; h++) {
-    const int i = 2 * tid + h;
-    kept[h] = i < n && (i == n - 1 || sk[i] != sk[i + 1]);
-    mine += kept[h];
-  }
-  int incl = mine;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if ((tid & 31) >= o) incl += y;
-  }
-  if ((tid & 31) == 31) wsum[tid >> 5] = incl;
-  __syncthreads();
-  int before = incl - mine;
-  for (int w = 0; w < (tid >> 5); w++) before += wsum[w];
-  for (int h = 0; h < 2; h++) {
-    const int i = 2 * tid + h;
-    if (kept[h]) {
-      bk[before] = (int64_t)(sk[i] ^ kSign);
-      if (bv) bv[before] = vals[si[i]];
-      before++;
+    const int64_t *r = t.inner + (int64_t)node * row;
+    const int32_t first = __ldg(t.prefix + node);
+    int k = 0;
+    for (int v = 0; v < ix / 2; v++) {
+      const longlong2 p = __ldg(reinterpret_cast<const longlong2 *>(r + 2 * v));
+      k += (p.x <= q) + (p.y <= q);
     }
+    k = min(k, ix - 1);
+    int c = 8 * k;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      const longlong2 p = __ldg(reinterpret_cast<const longlong2 *>(r + ix + 8 * k + 2 * v));
+      c += (p.x <= q) + (p.y <= q);
+    }
+    node = first + c;
   }
-  if (tid == blockDim.x - 1) *count = before;
+  return node - t.n_inner;
 }
 
-// ---- small epochs in one kernel ----
-//
-// An epoch of at most kSmallEpoch keys (the serving loop's write requests)
-// whose new keys all fit their leaves is applied by one CTA: bitonic sort of
-// (key, input index) in shared memory, last occurrence kept, a descent per
-// key, hits written in place, each leaf's new keys merged into its sorted row
-// from the back; a second kernel adds the new keys to leaf_base.  The CTA
-// checks everything (Max_Key, room in every touched leaf) before it writes
-// anything, so an epoch it cannot apply leaves the tree untouched for the
-// general path.  Same results as the general path, one host synchronisation
-// instead of four.
-constexpr int kSmallEpoch = 1024;
+// Whether a set bit of mask before position i belongs to a key of the same
+// leaf as position i's.  (A leaf's keys are one run of the sorted batch.)
+__device__ __forceinline__ bool marked_before(const uint32_t *__restrict__ mask, const int32_t *__restrict__ leaf_of,
+                                              int64_t i, int32_t leaf) {
+  while (i > 0 && leaf_of[i - 1] == leaf) {
+    const int64_t w = (i - 1) >> 5;
+    const uint32_t m = mask[w] & (0xffffffffu >> (31 - ((i - 1) & 31)));
+    if (m) return leaf_of[w * 32 + 31 - __clz(m)] == leaf;
+    i = w * 32;
+  }
+  return false;
+}
 
-struct SmallEpochResult {
-  int32_t applied;   // 1: applied in place; 0: nothing changed
-  int32_t maxkey;    // a key equals Max_Key (nothing changed)
-  int32_t inserted;  // new keys
-  int32_t runs;      // leaves that received new keys
-  int64_t new_min, new_max;  // smallest and largest new key
+// First set bit of mask at or after i whose key lies in `leaf`; -1 if none.
+__device__ __forceinline__ int64_t next_marked(const uint32_t *__restrict__ mask, const int32_t *__restrict__ leaf_of,
+                                               int64_t i, int64_t n, int32_t leaf) {
+  while (i < n && leaf_of[i] == leaf) {
+    const uint32_t m = mask[i >> 5] >> (i & 31);
+    if (m) {
+      i += __ffs(m) - 1;
+      return leaf_of[i] == leaf ? i : -1;
+    }
+    i = (i | 31) + 1;
+  }
+  return -1;
+}
+
+// Up to 32 marked keys of the sorted batch that a warp works on.
+struct WarpRows {
+  int64_t key[32], val[32];  // by lane (upsert)
+  uint32_t members[32];      // the lanes of the r-th leaf
+  int32_t head[32];          // the first of them
 };
 
-__global__ void __launch_bounds__(kSmallEpoch) small_epoch_kernel(
-    DevTree t, int f, int lc, int li, int flags, const int64_t *__restrict__ keys, const int64_t *__restrict__ vals,
-    int n, int64_t *leaf_rows, int32_t *leaf_cnt, int32_t *__restrict__ run_leaf, int32_t *__restrict__ run_pre,
-    SmallEpochResult *__restrict__ res) {
-  __shared__ uint64_t sk[kSmallEpoch];
-  __shared__ int32_t si[kSmallEpoch];
-  __shared__ int64_t kk[kSmallEpoch], kv[kSmallEpoch];  // kept keys and values, key order
-  __shared__ int32_t lf[kSmallEpoch];                     // their leaves; then the misses' leaves
-  __shared__ int32_t wsum[32];
-  __shared__ int32_t total;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // exclusive block scan of one int per thread; total of all in `total`
-  auto scan = [&](int v) {
-    int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
+// The last leaf's new keys past the warp's 32.
+struct NextKeys {
+  int32_t leaf = -1;  // the last leaf
+  int64_t at = 0;     // where its other keys may follow
+  const uint32_t *mask = nullptr;
+  const int32_t *leaf_of = nullptr;
+  const int64_t *sk = nullptr;
+  const int32_t *spos = nullptr;
+  const int64_t *vals = nullptr;
+  int64_t n = 0;
+};
+
+// The rows of the nh listed leaves, by groups of LC / 4 lanes that hold four
+// slots each (eight 16-key leaves at a time).  Upsert: a leaf's new keys are
+// placed among the sorted ones; a leaf without room for all of them is left as
+// it is.  Delete: the emptied slots (Max_Key) are squeezed out in key order.
+// Adds the keys stored or removed to *changed (per lane).
+template <int LC, bool DEL>
+__device__ __forceinline__ void write_rows(WarpRows &wr, int nh, int32_t leaf, const NextKeys &nx,
+                                           int64_t *leaf_rows, int32_t *leaf_cnt, bsort::Ctl *ctl, int *changed) {
+  constexpr int LI = LC >= 32 ? LC / 8 : 0;
+  constexpr int ROW = LI + 2 * LC;
+  constexpr int G = LC / 4, NG = 32 / G;
+  const int lane = threadIdx.x & 31, g = lane & (G - 1);
+  for (int b = 0; b < nh; b += NG) {
+    const int hi = b + lane / G;
+    const bool act = hi < nh;
+    uint32_t todo = act ? wr.members[hi] : 0;
+    const int32_t lf = __shfl_sync(0xffffffffu, leaf, act ? wr.head[hi] : 0);
+    int64_t *kr = leaf_rows + (int64_t)lf * ROW + LI, *vr = kr + LC;
+    int64_t k[4], v[4];
+    int to[4];  // where the slot's record goes
+    {
+      const longlong2 a = *reinterpret_cast<const longlong2 *>(kr + 4 * g);
+      const longlong2 c = *reinterpret_cast<const longlong2 *>(kr + 4 * g + 2);
+      const longlong2 d = *reinterpret_cast<const longlong2 *>(vr + 4 * g);
+      const longlong2 e = *reinterpret_cast<const longlong2 *>(vr + 4 * g + 2);
+      k[0] = a.x, k[1] = a.y, k[2] = c.x, k[3] = c.y;
+      v[0] = d.x, v[1] = d.y, v[2] = e.x, v[3] = e.y;
     }
-    __syncthreads();
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    int before = incl - v;
-    for (int w = 0; w < warp; w++) before += wsum[w];
-    if (tid == blockDim.x - 1) total = before + v;
-    __syncthreads();
-    return before;
-  };
-  int P = 1;
-  while (P < n) P <<= 1;
-  bool mx = false;
-  for (int i = tid; i < P; i += blockDim.x) {
-    const bool real = i < n;
-    const int64_t k = real ? keys[i] : 0;
-    mx |= real && k == kMaxKey;
-    sk[i] = real ? (uint64_t)k ^ kSign : ~0ull;  // padding sorts after every real key
-    si[i] = real ? i : INT32_MAX;
-  }
-  if (__syncthreads_or(mx)) {
-    if (tid == 0) res->maxkey = 1;
-    return;
-  }
-  for (int k = 2; k <= P; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = tid; i < P; i += blockDim.x) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const bool asc = (i & k) == 0;
-          const bool gt = sk[i] > sk[ixj] || (sk[i] == sk[ixj] && si[i] > si[ixj]);
-          if (gt == asc) {
-            const uint64_t tk = sk[i];
-            sk[i] = sk[ixj];
-            sk[ixj] = tk;
-            const int32_t ti = si[i];
-            si[i] = si[ixj];
-            si[ixj] = ti;
+    const int cnt = leaf_cnt[lf];
+    bool used[4];
+#pragma unroll
+    for (int x = 0; x < 4; x++) used[x] = 4 * g + x < cnt;
+    if constexpr (DEL) {
+      int mine = 0;
+#pragma unroll
+      for (int x = 0; x < 4; x++) {
+        used[x] &= k[x] != kMaxKey;
+        mine += used[x];
+      }
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o, G);
+        if (g >= o) incl += y;
+      }
+      const int live = __shfl_sync(0xffffffffu, incl, G - 1, G);
+      int at = incl - mine;
+#pragma unroll
+      for (int x = 0; x < 4; x++) to[x] = used[x] ? at++ : -1;
+      __syncwarp();  // every lane has read its slots
+      if (act) {
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          const int s = 4 * g + x;
+          if (to[x] >= 0 && to[x] != s) {
+            kr[to[x]] = k[x];
+            vr[to[x]] = v[x];
+          }
+          if (s >= live && s < cnt) {
+            kr[s] = kMaxKey;
+            vr[s] = HM_NOT_FOUND;
           }
         }
+        if (g == 0) {
+          leaf_cnt[lf] = live;
+          *changed += cnt - live;
+          if (live == 0) ctl->user[kUserEmpty] = 1;
+        }
       }
-      __syncthreads();
-    }
-  }
-  // keep each key's last occurrence (thread i owns sorted element i)
-  const bool keep = tid < n && (tid == n - 1 || sk[tid] != sk[tid + 1]);
-  const int at = scan(keep);
-  const int m = total;
-  if (keep) {
-    kk[at] = (int64_t)(sk[tid] ^ kSign);
-    kv[at] = vals[si[tid]];
-  }
-  __syncthreads();
-  // descend: hit slot or miss, per kept key (thread i owns kept key i)
-  int64_t key = 0, val = 0;
-  int32_t leaf = -1, slot = -1;
-  const int stride = li + 2 * lc;
-  if (tid < m) {
-    key = kk[tid];
-    val = kv[tid];
-    leaf = descend_leaf(t, f, key);
-    const int64_t *kr = t.leaf_rows + (int64_t)leaf * stride + li;
-    const int cnt = t.leaf_cnt[leaf];
-    for (int x = 0; x < cnt; x++)
-      if (kr[x] == key) slot = x;
-  }
-  const bool miss = tid < m && slot < 0;
-  const int mi = scan(miss);
-  const int nm = total;
-  if (miss) {  // the misses, still in key order, compacted
-    kk[mi] = key;
-    kv[mi] = val;
-    lf[mi] = leaf;
-  }
-  __syncthreads();
-  // runs of misses per leaf, and room for each run
-  bool start = false, fits = true;
-  int rl = 0;
-  if (tid < nm) {
-    start = tid == 0 || lf[tid] != lf[tid - 1];
-    if (start) {
-      int e = tid + 1;
-      while (e < nm && lf[e] == lf[tid]) e++;
-      rl = e - tid;
-      fits = t.leaf_cnt[lf[tid]] + rl <= lc;
-    }
-  }
-  if (!__syncthreads_and(fits)) return;  // res->applied stays 0: nothing changed
-  // hits in place (before the merges, which move the rows' values)
-  if (tid < m && slot >= 0)
-    leaf_rows[(int64_t)leaf * stride + li + lc + slot] = (flags & HM_UPSERT_REF_KEY_MINUS_1) ? key - 1 : val;
-  __syncthreads();
-  const int r = scan(start);
-  const int runs = total;
-  if (start) {
-    // merge the run [tid, tid + rl) into the leaf's sorted row from the back
-    const int32_t L = lf[tid];
-    int64_t *kr = leaf_rows + (int64_t)L * stride + li;
-    int64_t *vr = kr + lc;
-    int a = leaf_cnt[L], b = rl;
-    for (int o = a + b - 1; o >= 0 && b > 0; o--) {
-      if (a > 0 && kr[a - 1] > kk[tid + b - 1]) {
-        kr[o] = kr[a - 1];
-        vr[o] = vr[a - 1];
-        a--;
-      } else {
-        kr[o] = kk[tid + b - 1];
-        vr[o] = kv[tid + b - 1];
-        b--;
-      }
-    }
-    const int nc = leaf_cnt[L] + rl;
-    if (li > 0) {
-      int64_t *ir = leaf_rows + (int64_t)L * stride;
-      for (int x = 0; x < li; x++) ir[x] = (8 * (x + 1) < nc) ? kr[8 * (x + 1)] : kMaxKey;
-    }
-    leaf_cnt[L] = nc;
-    run_leaf[r] = L;
-    run_pre[r] = tid;  // new keys in earlier runs (the misses before this run)
-  }
-  if (tid == 0) {
-    res->applied = 1;
-    res->inserted = nm;
-    res->runs = runs;
-    if (nm > 0) {
-      res->new_min = kk[0];
-      res->new_max = kk[nm - 1];
-    }
-  }
-}
-
-// leaf_base[l] += new keys in leaves before l, after an applied small epoch.
-__global__ void small_epoch_base_kernel(int64_t *leaf_base, int64_t n_leaf, const int32_t *__restrict__ run_leaf,
-                                        const int32_t *__restrict__ run_pre, const SmallEpochResult *__restrict__ res) {
-  if (!res->applied || res->inserted == 0) return;
-  const int runs = res->runs, inserted = res->inserted;
-  for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < n_leaf; l += (int64_t)gridDim.x * blockDim.x) {
-    int lo = 0, hi = runs;  // first run whose leaf >= l
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (run_leaf[mid] < l) lo = mid + 1; else hi = mid;
-    }
-    const int add = lo < runs ? run_pre[lo] : inserted;
-    if (add) leaf_base[l] += add;
-  }
-}
-
-// Hits are updated in place; misses get miss[i] = 1 and their leaf.
-__global__ void apply_kernel(DevTree t, int f, int lc, int li, int flags,
-                             const int64_t *__restrict__ bk, const int64_t *__restrict__ bv, int64_t m,
-                             int64_t *leaf_rows, int32_t *__restrict__ miss,
-                             int32_t *__restrict__ leaf_of) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t k = bk[i];
-    int32_t leaf = descend_leaf(t, f, k);
-    const int64_t *kr = t.leaf_rows + (int64_t)leaf * (li + 2 * lc) + li;
-    int cnt = t.leaf_cnt[leaf];
-    int slot = -1;
-    for (int s = 0; s < cnt; s++)
-      if (kr[s] == k) slot = s;
-    leaf_of[i] = leaf;
-    if (slot >= 0) {
-      leaf_rows[(int64_t)leaf * (li + 2 * lc) + li + lc + slot] =
-          (flags & HM_UPSERT_REF_KEY_MINUS_1) ? k - 1 : bv[i];
-      miss[i] = 0;
     } else {
-      miss[i] = 1;
+      int64_t nk[4], nv[4];
+      int ns[4], m = 0;
+#pragma unroll
+      for (int x = 0; x < 4; x++) {
+        to[x] = 4 * g + x;
+        ns[x] = -1;
+      }
+      bool on = act && lf == nx.leaf, over = false;  // its run may go on
+      int64_t at = nx.at;
+      while (__any_sync(0xffffffffu, todo != 0 || on)) {
+        int64_t q = 0, val = 0;
+        bool have = todo != 0;
+        if (have) {
+          const int j = __ffs(todo) - 1;
+          todo &= todo - 1;
+          q = wr.key[j];
+          val = wr.val[j];
+        } else if (on) {
+          at = next_marked(nx.mask, nx.leaf_of, at, nx.n, lf);
+          on = have = at >= 0;
+          if (have) {
+            q = nx.sk[at];
+            val = nx.vals[nx.spos[at]];
+            at++;
+          }
+        }
+        if (have && cnt + m == LC) {  // no room
+          over = true;
+          have = on = false;
+          todo = 0;
+        }
+        int below = 0;
+#pragma unroll
+        for (int x = 0; x < 4; x++) below += have && used[x] && k[x] < q;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+        if (have) {
+#pragma unroll
+          for (int x = 0; x < 4; x++) {
+            to[x] += used[x] && k[x] > q;
+            if (4 * g + x == m) {  // the lane of slot m keeps the m-th new key
+              nk[x] = q;
+              nv[x] = val;
+              ns[x] = below + m;
+            }
+          }
+          m++;
+        }
+      }
+      __syncwarp();  // every lane has read its slots
+      if (act && !over) {
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          if (used[x] && to[x] != 4 * g + x) {
+            kr[to[x]] = k[x];
+            vr[to[x]] = v[x];
+          }
+          if (ns[x] >= 0) {
+            kr[ns[x]] = nk[x];
+            vr[ns[x]] = nv[x];
+          }
+        }
+        if (g == 0) {
+          leaf_cnt[lf] = cnt + m;
+          *changed += m;
+        }
+      }
+      if (over && g == 0) ctl->user[kUserOverflow] = 1;
     }
+    if constexpr (LI > 0) {
+      __syncwarp();
+      if (act && g < LI) kr[g - LI] = 8 * (g + 1) < LC ? kr[8 * (g + 1)] : kMaxKey;
+    }
+  }
+  __syncwarp();
+}
+
+// The batch against the leaves: a warp takes 32 neighbouring keys of the
+// sorted batch, finds their leaves, and looks each key up in its leaf with
+// four lanes (all 32 leaves' loads are issued before the first is used).
+// Upsert: the last of equal keys counts; a stored key's value is overwritten
+// (supplied value, or key - 1 under HM_UPSERT_REF_KEY_MINUS_1), a new key sets
+// its bit in mask.  Delete: a stored key's slot becomes Max_Key and its bit is
+// set.  leaf_of gets every key's leaf.  Nothing happens if a key of an upsert
+// is Max_Key.
+//
+// Bound by DRAM on scattered sectors: a key's 128-B key row, the sector its
+// value is written to and its value's sector.  Launched in full after the
+// sort, not as a dependent launch: an SM keeps the shared-memory carve-out of
+// the CTAs it runs, and CTAs that start behind the sort's would run the whole
+// kernel with the little L1 the sort leaves (4096K keys on 2^26: 277 against
+// 200 us).
+template <int LC, bool DEL>
+__global__ void __launch_bounds__(kApply, 10) apply_kernel(DevTree t, int f, int flags, const int64_t *__restrict__ sk,
+                                                         const int32_t *__restrict__ spos,
+                                                         const int64_t *__restrict__ vals, int64_t n,
+                                                         int64_t *leaf_rows, int32_t *__restrict__ leaf_of,
+                                                         uint32_t *__restrict__ mask, bsort::Ctl *ctl,
+                                                         const unsigned *__restrict__ err) {
+  constexpr int LI = LC >= 32 ? LC / 8 : 0;
+  constexpr int ROW = LI + 2 * LC;
+  const int lane = threadIdx.x & 31;
+  const int64_t word = blockIdx.x * (int64_t)(kApply / 32) + (threadIdx.x >> 5), w0 = word * 32;
+  if (w0 >= n) return;
+  const int64_t i = min(w0 + lane, n - 1);
+  const int64_t key = __ldg(sk + i);
+  bool live = w0 + lane < n;
+  int32_t pos = 0;
+  int64_t val = 0;
+  if constexpr (DEL) {
+    live &= key != kMaxKey;  // never stored
+  } else {
+    live &= i == n - 1 || __ldg(sk + min(i + 1, n - 1)) != key;
+    pos = __ldg(spos + i);
+  }
+  if (ctl->skew || (!DEL && (ctl->flags & 2u))) return;
+  if (word == 0 && lane == 0) ctl->user[kUserErr] = *err;
+  const int32_t leaf = descend_leaf_warp(t, f, DEL && key == kMaxKey ? kMaxKey - 1 : key);
+  if (w0 + lane < n) leaf_of[i] = leaf;
+  // four lanes per key, eight keys per step
+  const int sub = lane & 3;
+  longlong2 a[4], b[4];
+  int base[4];
+#pragma unroll
+  for (int s = 0; s < 4; s++) {
+    const int32_t lf = __shfl_sync(0xffffffffu, leaf, s * 8 + (lane >> 2));
+    const int64_t *r = leaf_rows + (int64_t)lf * ROW;
+    base[s] = 0;
+    if constexpr (LI == 0) {
+      a[s] = *reinterpret_cast<const longlong2 *>(r + 2 * sub);
+      b[s] = *reinterpret_cast<const longlong2 *>(r + 8 + 2 * sub);
+    } else {
+      a[s] = *reinterpret_cast<const longlong2 *>(r + 2 * sub);  // the leaf's index words
+    }
+  }
+  if constexpr (!DEL) val = flags & HM_UPSERT_REF_KEY_MINUS_1 ? key - 1 : __ldg(vals + pos);
+  if constexpr (LI != 0) {
+    static_assert(LI == 0 || LI == 8, "two index words a lane");
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+      const int64_t q = __shfl_sync(0xffffffffu, key, s * 8 + (lane >> 2));
+      int k = (a[s].x <= q) + (a[s].y <= q);
+      k += __shfl_xor_sync(0xffffffffu, k, 1);
+      k += __shfl_xor_sync(0xffffffffu, k, 2);
+      base[s] = 8 * min(k, LI - 1);
+      const int32_t lf = __shfl_sync(0xffffffffu, leaf, s * 8 + (lane >> 2));
+      a[s] = *reinterpret_cast<const longlong2 *>(leaf_rows + (int64_t)lf * ROW + LI + base[s] + 2 * sub);
+      b[s] = make_longlong2(0, 0);
+    }
+  }
+  const uint32_t lives = __ballot_sync(0xffffffffu, live);
+  bool hit = false;
+#pragma unroll
+  for (int s = 0; s < 4; s++) {
+    const int own = s * 8 + (lane >> 2);
+    const int64_t q = __shfl_sync(0xffffffffu, key, own);
+    const int32_t lf = __shfl_sync(0xffffffffu, leaf, own);
+    const int64_t v = __shfl_sync(0xffffffffu, val, own);
+    int slot = -1;
+    if constexpr (LI == 0) {
+      if (a[s].x == q) slot = 2 * sub;
+      if (a[s].y == q) slot = 2 * sub + 1;
+      if (b[s].x == q) slot = 8 + 2 * sub;
+      if (b[s].y == q) slot = 8 + 2 * sub + 1;
+    } else {
+      if (a[s].x == q) slot = base[s] + 2 * sub;
+      if (a[s].y == q) slot = base[s] + 2 * sub + 1;
+    }
+    if (!((lives >> own) & 1u)) slot = -1;
+    if (slot >= 0) {
+      int64_t *r = leaf_rows + (int64_t)lf * ROW + LI + slot;
+      if constexpr (DEL)
+        r[0] = kMaxKey;
+      else
+        r[LC] = v;
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, slot >= 0);
+    if (lane >> 3 == s) hit = (m >> (4 * (lane & 7))) & 0xfu;
+  }
+  const uint32_t out = __ballot_sync(0xffffffffu, live && (DEL ? hit : !hit));
+  if (lane == 0) mask[word] = out;
+}
+
+// Position of the k-th set bit of w (k < __popc(w)).
+__device__ __forceinline__ int nth_bit(uint32_t w, int k) {
+  int at = 0;
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1) {
+    const int c = __popc((w >> at) & ((1u << step) - 1u));
+    if (k >= c) {
+      k -= c;
+      at += step;
+    }
+  }
+  return at;
+}
+
+// The rows of the leaves of the marked keys.  A warp takes wpw words of the
+// mask (few in a small batch, for more warps) and their marked keys 32 at a
+// time, one per lane, so that their loads are in flight together; a leaf is
+// handled where its first marked key lies.
+template <int LC, bool DEL>
+__global__ void __launch_bounds__(kRowThreads) leaf_rows_kernel(const int64_t *__restrict__ sk,
+                                                                const int32_t *__restrict__ spos,
+                                                                const int64_t *__restrict__ vals, int64_t n, int wpw,
+                                                                const int32_t *__restrict__ leaf_of,
+                                                                const uint32_t *__restrict__ mask, int64_t *leaf_rows,
+                                                                int32_t *leaf_cnt, bsort::Ctl *ctl) {
+  pdl_enter();
+  __shared__ WarpRows s_rows[kRowThreads / 32];
+  if (ctl->skew || (!DEL && (ctl->flags & 2u))) return;
+  const int lane = threadIdx.x & 31;
+  WarpRows &wr = s_rows[threadIdx.x >> 5];
+  const int64_t words = (n + 31) / 32;
+  const int64_t base = (blockIdx.x * (int64_t)(kRowThreads / 32) + (threadIdx.x >> 5)) * wpw;
+  const uint32_t mine = lane < wpw && base + lane < words ? mask[base + lane] : 0;
+  const int cnt = __popc(mine);
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  int changed = 0;
+  int32_t last = -1;  // leaf of the last marked key of the round before
+  for (int c0 = 0; c0 < total; c0 += 32) {
+    const int r = min(c0 + lane, total - 1);
+    const bool valid = c0 + lane < total;
+    int wl = 0;  // the lane whose word holds marked key r
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, wl + step - 1) <= r) wl += step;
+    const uint32_t w = __shfl_sync(0xffffffffu, mine, wl);
+    const int below = __shfl_sync(0xffffffffu, incl - cnt, wl);
+    const int64_t i = (base + wl) * 32 + nth_bit(w, r - below);
+    const int32_t leaf = leaf_of[i];
+    if (!DEL) {
+      wr.key[lane] = sk[i];
+      wr.val[lane] = vals[spos[i]];
+    }
+    const int32_t up = __shfl_up_sync(0xffffffffu, leaf, 1);
+    bool head = valid && leaf != (lane == 0 ? last : up);
+    if (c0 == 0 && lane == 0) head = !marked_before(mask, leaf_of, i, leaf);
+    const uint32_t heads = __ballot_sync(0xffffffffu, head);
+    const uint32_t members = __match_any_sync(0xffffffffu, leaf) & __ballot_sync(0xffffffffu, valid);
+    if (head) {
+      const int h = __popc(heads & ((1u << lane) - 1u));
+      wr.head[h] = lane;
+      wr.members[h] = members;
+    }
+    last = __shfl_sync(0xffffffffu, leaf, 31);
+    NextKeys nx;
+    if (!DEL) nx = NextKeys{last, __shfl_sync(0xffffffffu, i, 31) + 1, mask, leaf_of, sk, spos, vals, n};
+    __syncwarp();
+    write_rows<LC, DEL>(wr, __popc(heads), leaf, nx, leaf_rows, leaf_cnt, ctl, &changed);
+  }
+  changed = __reduce_add_sync(0xffffffffu, changed);
+  if (lane == 0 && changed > 0) atomicAdd(&ctl->user[kUserChanged], (unsigned long long)changed);
+}
+
+// New keys that their leaf had no room for, as flags to scan.
+__global__ void left_over_kernel(const int64_t *__restrict__ sk, const int32_t *__restrict__ leaf_of,
+                                 const uint32_t *__restrict__ mask, int64_t n, int lc, int li,
+                                 const int64_t *__restrict__ leaf_rows, int32_t *__restrict__ miss) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    bool left = (mask[i >> 5] >> (i & 31)) & 1u;
+    if (left) {
+      const int64_t q = sk[i];
+      const int64_t *kr = leaf_rows + (int64_t)leaf_of[i] * (li + 2 * lc) + li;
+      for (int s = 0; s < lc; s++) left &= kr[s] != q;
+    }
+    miss[i] = left;
   }
 }
 
-__global__ void compact_miss_kernel(const int64_t *__restrict__ bk, const int64_t *__restrict__ bv,
-                                    const int32_t *__restrict__ leaf_of, const int32_t *__restrict__ miss,
-                                    const int64_t *__restrict__ at, int64_t m, int64_t *__restrict__ mk,
-                                    int64_t *__restrict__ mv, int32_t *__restrict__ ml) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
+__global__ void compact_miss_kernel(const int64_t *__restrict__ sk, const int32_t *__restrict__ spos,
+                                    const int64_t *__restrict__ vals, const int32_t *__restrict__ leaf_of,
+                                    const int32_t *__restrict__ miss, const int64_t *__restrict__ at, int64_t n,
+                                    int64_t *__restrict__ mk, int64_t *__restrict__ mv, int32_t *__restrict__ ml) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     if (miss[i]) {
       int64_t o = at[i];
-      mk[o] = bk[i];
-      mv[o] = bv[i];
+      mk[o] = sk[i];
+      mv[o] = vals[spos[i]];
       ml[o] = leaf_of[i];
     }
   }
 }
 
-// For each run of misses on one leaf (misses are in key order, so leaves are
-// non-decreasing): seg_start[leaf] = first miss index, add[leaf] = run length;
-// flags bit0 if the leaf would overflow.
-__global__ void miss_runs_kernel(const int32_t *__restrict__ ml, int64_t nm,
-                                 const int32_t *__restrict__ leaf_cnt, int lc,
-                                 int64_t *__restrict__ run_start, int32_t *__restrict__ run_len,
-                                 int32_t *__restrict__ run_leaf, int32_t *__restrict__ is_start,
-                                 unsigned *flags) {
+// For each run of left-over keys on one leaf (they are in key order, so
+// leaves are non-decreasing): its first key is marked and gets the run's
+// length and leaf.
+__global__ void miss_runs_kernel(const int32_t *__restrict__ ml, int64_t nm, int32_t *__restrict__ run_len,
+                                 int32_t *__restrict__ run_leaf, int32_t *__restrict__ is_start) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nm;
        i += (int64_t)gridDim.x * blockDim.x) {
     bool st = (i == 0) || ml[i] != ml[i - 1];
@@ -392,64 +590,9 @@ __global__ void miss_runs_kernel(const int32_t *__restrict__ ml, int64_t nm,
     if (st) {
       int64_t e = i + 1;
       while (e < nm && ml[e] == ml[i]) e++;
-      run_start[i] = i;
       run_len[i] = (int32_t)(e - i);
       run_leaf[i] = ml[i];
-      if (leaf_cnt[ml[i]] + (e - i) > lc) atomicOr(flags, 1u);
     }
-  }
-}
-
-// One warp per run: merge the run's new keys into the leaf row.
-__global__ void merge_leaf_kernel(int64_t *leaf_rows, int32_t *leaf_cnt, int lc,
-                                  int li, const int64_t *__restrict__ mk, const int64_t *__restrict__ mv,
-                                  const int32_t *__restrict__ is_start,
-                                  const int64_t *__restrict__ run_start,
-                                  const int32_t *__restrict__ run_len,
-                                  const int32_t *__restrict__ run_leaf, int64_t nm,
-                                  const int32_t *__restrict__ run_parent = nullptr,
-                                  const int32_t *__restrict__ mark = nullptr) {
-  __shared__ int64_t sk[kThreads / 32][128];
-  __shared__ int64_t sv[kThreads / 32][128];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
-  for (int64_t i = blockIdx.x * (int64_t)(blockDim.x / 32) + w; i < nm; i += warps) {
-    if (!is_start[i]) continue;
-    if (mark && mark[run_parent[i]]) continue;  // its subtree is rebalanced instead
-    const int32_t leaf = run_leaf[i];
-    const int64_t r0 = run_start[i];
-    const int rl = run_len[i];
-    int64_t *kr = leaf_rows + (int64_t)leaf * (li + 2 * lc) + li;
-    int64_t *vr = kr + lc;
-    const int cnt = leaf_cnt[leaf];
-    // existing key a goes to a + #(new < key); new key b to b + #(existing < key)
-    for (int a = lane; a < cnt; a += 32) {
-      int64_t k = kr[a];
-      int below = 0;
-      for (int b = 0; b < rl; b++) below += (mk[r0 + b] < k);
-      sk[w][a + below] = k;
-      sv[w][a + below] = vr[a];
-    }
-    for (int b = lane; b < rl; b += 32) {
-      int64_t k = mk[r0 + b];
-      int below = 0;
-      for (int a = 0; a < cnt; a++) below += (kr[a] < k);
-      sk[w][b + below] = k;
-      sv[w][b + below] = mv[r0 + b];
-    }
-    __syncwarp();
-    const int nc = cnt + rl;
-    for (int x = lane; x < lc; x += 32) {
-      kr[x] = x < nc ? sk[w][x] : kMaxKey;
-      vr[x] = x < nc ? sv[w][x] : (int64_t)HM_NOT_FOUND;
-    }
-    __syncwarp();
-    if (li > 0) {
-      int64_t *ir = leaf_rows + (int64_t)leaf * (li + 2 * lc);
-      for (int x = lane; x < li; x += 32) ir[x] = (8 * (x + 1) < lc) ? kr[8 * (x + 1)] : kMaxKey;
-    }
-    if (lane == 0) leaf_cnt[leaf] = nc;
-    __syncwarp();
   }
 }
 
@@ -611,66 +754,127 @@ __global__ void merge_rank_kernel(const int64_t *__restrict__ a, const int64_t *
   }
 }
 
-// ---- delete epochs ----
-
-__global__ void compact_keys_kernel(const uint64_t *__restrict__ uk, const int32_t *__restrict__ keep,
-                                    const int64_t *__restrict__ at, int64_t n, int64_t *__restrict__ bk) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    if (keep[i]) bk[at[i]] = (int64_t)(uk[i] ^ kSign);
-}
-
-// One thread per distinct key: descend; a stored key's slot is overwritten
-// with Max_Key (the leaf is compacted next); route[i] = the key's leaf.
-__global__ void delete_mark_kernel(DevTree t, int f, int lc, int li, const int64_t *__restrict__ bk, int64_t m,
-                                   int64_t *leaf_rows, int32_t *__restrict__ route) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = bk[i];
-    const int32_t leaf = descend_leaf(t, f, k == kMaxKey ? kMaxKey - 1 : k);  // never rank the sentinel
-    route[i] = leaf;
-    if (k == kMaxKey) continue;  // never stored
-    int64_t *kr = leaf_rows + (int64_t)leaf * (li + 2 * lc) + li;
-    const int cnt = t.leaf_cnt[leaf];
-    for (int s = 0; s < cnt; s++)
-      if (kr[s] == k) kr[s] = kMaxKey;
-  }
-}
-
-// One thread per leaf the batch routed to (keys are sorted, so each leaf's
-// keys are one run of route[]): squeeze out the marked slots keeping key
-// order, refresh the leaf index words, count what went; flags bit0 when a
-// leaf that held keys is left empty (the tree is then rebuilt).
-__global__ void delete_compact_kernel(int64_t *leaf_rows, int32_t *leaf_cnt, int lc, int li,
-                                      const int32_t *__restrict__ route, int64_t m,
-                                      unsigned long long *removed, unsigned *flags) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    if (i > 0 && route[i - 1] == route[i]) continue;
-    const int32_t leaf = route[i];
-    int64_t *row = leaf_rows + (int64_t)leaf * (li + 2 * lc);
-    int64_t *kr = row + li, *vr = kr + lc;
-    const int cnt = leaf_cnt[leaf];
-    int live = 0;
-    for (int s = 0; s < cnt; s++) {
-      if (kr[s] == kMaxKey) continue;
-      kr[live] = kr[s];
-      vr[live] = vr[s];
-      live++;
-    }
-    if (live == cnt) continue;
-    for (int s = live; s < cnt; s++) {
-      kr[s] = kMaxKey;
-      vr[s] = HM_NOT_FOUND;
-    }
-    for (int x = 0; x < li; x++) row[x] = (8 * (x + 1) < lc) ? kr[8 * (x + 1)] : kMaxKey;
-    leaf_cnt[leaf] = live;
-    atomicAdd(removed, (unsigned long long)(cnt - live));
-    if (live == 0) atomicOr(flags, 1u);
-  }
-}
-
 size_t al(int64_t bytes) { return (size_t)align_up(bytes, 256); }
+
+// Keys in one upsert or delete epoch, at most: the batch sort carries each
+// key's input position as an int32 (such a batch would need about 200 GB of
+// scratch anyway).
+constexpr int64_t kMaxEpochKeys = 0x7fffffff;
+
+// A batch in key order on its way through the tree (device memory of one
+// scratch lease).
+struct Epoch {
+  int64_t n = 0;
+  int64_t *ka = nullptr, *kb = nullptr;  // sort buffers; the sorted keys end in sk
+  int32_t *pa = nullptr, *pb = nullptr;
+  int64_t *sk = nullptr;
+  int32_t *spos = nullptr;
+  int32_t *leaf_of = nullptr;
+  uint32_t *mask = nullptr;
+  void *sort_scratch = nullptr, *scan_scratch = nullptr;
+  bsort::Ctl *ctl = nullptr;
+
+  static size_t sort_bytes(int64_t n) {
+    return std::max(al((int64_t)radix_scratch_bytes(n)), bsort::fits(n) ? bsort::work_bytes(n) : 0) +
+           al(sizeof(bsort::Ctl));
+  }
+  static size_t scan_bytes(const hm_tree *t, int64_t n) {
+    return al((int64_t)scan_scratch_bytes(std::max<int64_t>(n, t->n_leaf) + 1));
+  }
+  static size_t bytes(const hm_tree *t, int64_t n) {
+    return 2 * al(8 * n) + 3 * al(4 * n) + al(4 * (n / 32 + 1)) + sort_bytes(n) + scan_bytes(t, n);
+  }
+  char *place(const hm_tree *t, int64_t n_, char *p) {
+    n = n_;
+    auto take = [&](size_t b) { char *r = p; p += b; return r; };
+    ka = reinterpret_cast<int64_t *>(take(al(8 * n)));
+    kb = reinterpret_cast<int64_t *>(take(al(8 * n)));
+    pa = reinterpret_cast<int32_t *>(take(al(4 * n)));
+    pb = reinterpret_cast<int32_t *>(take(al(4 * n)));
+    leaf_of = reinterpret_cast<int32_t *>(take(al(4 * n)));
+    mask = reinterpret_cast<uint32_t *>(take(al(4 * (n / 32 + 1))));
+    sort_scratch = take(sort_bytes(n));
+    scan_scratch = take(scan_bytes(t, n));
+    return p;
+  }
+
+  // Bucket sort of the batch; enqueues only.  The control block's skew says
+  // whether the batch's keys crowd a bucket, nothing was sorted then.
+  void bucket_sort(const hm_tree *t, const int64_t *keys, cudaStream_t s) {
+    const bsort::Work w = bsort::layout(n, sort_scratch);
+    ctl = w.ctl;
+    const int passes = bsort::partition_pairs<int32_t>(keys, nullptr, n, ka, pa, kb, pb, w, t->num_sms, s);
+    const int64_t *in_k = passes == 2 ? kb : passes == 1 ? ka : keys;
+    const int32_t *in_p = passes == 2 ? pb : passes == 1 ? pa : nullptr;
+    sk = passes == 1 ? kb : ka;
+    spos = passes == 1 ? pb : pa;
+    constexpr int sm = (int)sizeof(bsort::SortSmem<int32_t>);
+    opt_in_smem((const void *)epoch_sort_kernel, sm);
+    launch_pdl(epoch_sort_kernel, 1u << bsort::shape_for(n).bits, bsort::kSortThreads, sm, s, in_k, in_p,
+               static_cast<const uint32_t *>(passes ? w.start : nullptr), (uint32_t)n, sk, spos, ctl);
+    note_launch();
+  }
+
+  // LSD sort of the batch, for keys that the bucket sort does not take.
+  void lsd_sort(const int64_t *keys, cudaStream_t s) {
+    ctl = reinterpret_cast<bsort::Ctl *>(static_cast<char *>(sort_scratch) + al((int64_t)radix_scratch_bytes(n)));
+    cudaMemsetAsync(ctl, 0, sizeof(bsort::Ctl), s);
+    uint64_t *u = reinterpret_cast<uint64_t *>(ka), *ua = reinterpret_cast<uint64_t *>(kb);
+    transform_keys_in(keys, u, n, s);
+    const bool alt = radix_sort_positions(u, pa, ua, pb, n, 0, 64, sort_scratch, s);
+    sk = alt ? ka : kb;
+    spos = alt ? pb : pa;
+    lsd_finish_kernel<<<grid_for(n), kThreads, 0, s>>>(alt ? ua : u, n, sk, ctl);
+    note_launch();
+  }
+
+  // The sorted batch against the tree's leaves, and leaf_base after it.
+  void apply(const hm_tree *t, const int64_t *vals, int flags, bool del, cudaStream_t s) {
+    const unsigned key_grid = (unsigned)((n + kApply - 1) / kApply);
+    const int64_t words = (n + 31) / 32;
+    const int wpw = (int)std::min<int64_t>(32, std::max<int64_t>(1, words / (t->num_sms * 16)));
+    const unsigned row_grid = (unsigned)((words + wpw * (kRowThreads / 32) - 1) / (wpw * (kRowThreads / 32)));
+    const bool wide = t->cfg.leaf_cap != 16;
+    const int64_t *csk = sk;
+    const int32_t *cpos = spos, *cleaf = leaf_of;
+    const uint32_t *cmask = mask;
+    const unsigned *err = t->d_err;
+    auto look = del ? (wide ? apply_kernel<64, true> : apply_kernel<16, true>)
+                    : (wide ? apply_kernel<64, false> : apply_kernel<16, false>);
+    look<<<key_grid, kApply, 0, s>>>(t->view(), t->cfg.fanout, flags, csk, cpos, vals, n, t->leaf_rows, leaf_of, mask,
+                                     ctl, err);
+    auto rows = del ? (wide ? leaf_rows_kernel<64, true> : leaf_rows_kernel<16, true>)
+                    : (wide ? leaf_rows_kernel<64, false> : leaf_rows_kernel<16, false>);
+    launch_pdl(rows, row_grid, kRowThreads, 0, s, csk, cpos, vals, n, wpw, cleaf, cmask, t->leaf_rows, t->leaf_cnt,
+               ctl);
+    note_launch(2);
+    rescan_leaf_base(t, &ctl->user[kUserChanged], scan_scratch, s);
+  }
+
+  int run(const hm_tree *t, const int64_t *keys, const int64_t *vals, int flags, bool del, bsort::Ctl *h,
+          cudaStream_t s) {
+    h->skew = 1;
+    if (bsort::fits(n)) {
+      bucket_sort(t, keys, s);
+      apply(t, vals, flags, del, s);
+      int rc = read(h, s);
+      if (rc) return rc;
+    }
+    if (h->skew) {
+      lsd_sort(keys, s);
+      apply(t, vals, flags, del, s);
+      return read(h, s);
+    }
+    return HM_OK;
+  }
+
+  int read(bsort::Ctl *h, cudaStream_t s) const {
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, ctl, sizeof(*h), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    return cuda_err(e);
+  }
+};
 
 }  // namespace
 
@@ -698,7 +902,6 @@ int rebuild_from_sorted(hm_tree *t, const uint64_t *ck, const int64_t *cv, int64
   int64_t *tmp_a = reinterpret_cast<int64_t *>(tmp);
   int64_t *tmp_b = reinterpret_cast<int64_t *>(tmp + al(8 * tn));
   char *base = static_cast<char *>(arena);
-  cudaMemsetAsync(base, 0, total, s);
   nt.inner = reinterpret_cast<int64_t *>(base);
   nt.prefix = reinterpret_cast<int32_t *>(base + off_prefix);
   nt.leaf_rows = reinterpret_cast<int64_t *>(base + off_lrows);
@@ -730,279 +933,127 @@ int rebuild_from_sorted(hm_tree *t, const uint64_t *ck, const int64_t *cv, int64
   return HM_OK;
 }
 
-int upsert_epoch(hm_tree *t, const int64_t *d_keys, const int64_t *d_vals, int64_t n, int flags,
+int upsert_epoch(hm_tree *t, const int64_t *d_keys, const int64_t *d_vals, int64_t n, int flags, unsigned *err,
                  cudaStream_t s) {
   if (n <= 0) return HM_OK;
   if (n > kMaxEpochKeys) return HM_ETOOLARGE;
-  const int lc = t->cfg.leaf_cap, li = t->leaf_index, f = t->cfg.fanout;
-  if (n <= kSmallEpoch && t->n_keys > 0) {  // one kernel, one synchronisation, if every new key fits
-    ScratchLease lease(t, s);
-    const size_t rb = al(4 * n);
-    int rc = lease.acquire(2 * rb + al(sizeof(SmallEpochResult)) + 256);
-    if (rc) return rc;
-    char *p = static_cast<char *>(lease.ptr());
-    int32_t *run_leaf = reinterpret_cast<int32_t *>(p);
-    int32_t *run_pre = reinterpret_cast<int32_t *>(p + rb);
-    SmallEpochResult *dres = reinterpret_cast<SmallEpochResult *>(p + 2 * rb);
-    SmallEpochResult hres{};
-    cudaError_t e = cudaMemsetAsync(dres, 0, sizeof(SmallEpochResult), s);
-    if (e != cudaSuccess) return cuda_err(e);
-    small_epoch_kernel<<<1, kSmallEpoch, 0, s>>>(t->view(), f, lc, li, flags, d_keys, d_vals, (int)n, t->leaf_rows,
-                                                 t->leaf_cnt, run_leaf, run_pre, dres);
-    small_epoch_base_kernel<<<grid_for(t->n_leaf), kThreads, 0, s>>>(t->leaf_base, t->n_leaf, run_leaf, run_pre,
-                                                                     dres);
-    note_launch(2);
-    e = cudaMemcpyAsync(&hres, dres, sizeof(hres), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_err(e);
-    if (hres.maxkey) return HM_EMAXKEY;
-    if (hres.applied) {
-      t->n_keys += hres.inserted;
-      if (hres.inserted > 0) {
-        if (hres.new_min < t->key_min) t->key_min = hres.new_min;
-        if (hres.new_max > t->key_max) t->key_max = hres.new_max;
-      }
-      return HM_OK;
-    }
-    // some leaf has no room: nothing was changed; the general path below
-  }
-  // scratch: uk, uk_alt, idx, idx_alt (n each, 8 B), keep/miss/leaf_of/is_start (4 B),
-  // at (8 B, n+1), bk, bv, mk, mv, run_start (8 B), run_len/run_leaf/ml (4 B), sort scratch, flags
+  const int lc = t->cfg.leaf_cap, li = t->leaf_index;
+  // the batch's own memory, then what an epoch with overflowing leaves needs:
+  // at, mk, mv (8 B), miss, ml, is_start, run_len, run_leaf, run_parent (4 B)
+  // and the subtree marks, one per last-level node
   const size_t s8 = al(8 * (n + 1)), s4 = al(4 * (n + 1));
-  // the leaf_base rescan covers every leaf, not just the batch
-  const int64_t scan_n = std::max<int64_t>(n, t->n_leaf) + 1;
-  const size_t lb8 = al(8 * (t->n_leaf + 1));
-  const size_t mk4 = al(4 * (t->n_inner + 1));  // subtree marks, one per last-level node
-  size_t need = 9 * s8 + 7 * s4 + lb8 + mk4 + al((int64_t)radix_scratch_bytes(n)) +
-                al((int64_t)scan_scratch_bytes(scan_n)) + 256;
   ScratchLease lease(t, s);
-  int rc = lease.acquire(need);
+  int rc = lease.acquire(Epoch::bytes(t, n) + 3 * s8 + 6 * s4 + al(4 * (t->n_inner + 1)));
   if (rc) return rc;
-  char *p = static_cast<char *>(lease.ptr());
-  auto take8 = [&](void) { char *r = p; p += s8; return r; };
-  auto take4 = [&](void) { char *r = p; p += s4; return r; };
-  uint64_t *uk = reinterpret_cast<uint64_t *>(take8());
-  uint64_t *uk_alt = reinterpret_cast<uint64_t *>(take8());
-  int32_t *idx = reinterpret_cast<int32_t *>(take8());  // input positions (8-B slots: run_start reuses one)
-  int32_t *idx_alt = reinterpret_cast<int32_t *>(take8());
-  int64_t *at = reinterpret_cast<int64_t *>(take8());
-  int64_t *bk = reinterpret_cast<int64_t *>(take8());
-  int64_t *bv = reinterpret_cast<int64_t *>(take8());
-  int64_t *mk = reinterpret_cast<int64_t *>(take8());
-  int64_t *mv = reinterpret_cast<int64_t *>(take8());
-  int32_t *keep = reinterpret_cast<int32_t *>(take4());
-  int32_t *miss = reinterpret_cast<int32_t *>(take4());
-  int32_t *leaf_of = reinterpret_cast<int32_t *>(take4());
-  int32_t *ml = reinterpret_cast<int32_t *>(take4());
-  int32_t *is_start = reinterpret_cast<int32_t *>(take4());
-  int32_t *run_len = reinterpret_cast<int32_t *>(take4());
-  int32_t *run_leaf = reinterpret_cast<int32_t *>(take4());
-  int64_t *run_start = nullptr;  // the position buffer the sort leaves free
-  void *sort_scratch = p;
-  p += al((int64_t)radix_scratch_bytes(n));
-  int64_t *lbase_tmp = reinterpret_cast<int64_t *>(p);  // n_leaf + 1 entries
-  p += lb8;
-  void *scan_scratch = p;
-  p += al((int64_t)scan_scratch_bytes(scan_n));
-  int32_t *marks = reinterpret_cast<int32_t *>(p);
-  p += mk4;
-  unsigned *dflags = reinterpret_cast<unsigned *>(p);
+  Epoch ep;
+  char *p = ep.place(t, n, static_cast<char *>(lease.ptr()));
+  bsort::Ctl h{};
+  rc = ep.run(t, d_keys, d_vals, flags, false, &h, s);
+  if (rc) return rc;
+  if (h.flags & 2u) return HM_EMAXKEY;
+  *err = (unsigned)h.user[kUserErr];
+  const bool was_empty = t->n_keys == 0;
+  t->n_keys += (int64_t)h.user[kUserChanged];
+  // a stored key lies between key_min and key_max already
+  if (was_empty || h.ends[0] < t->key_min) t->key_min = h.ends[0];
+  if (was_empty || h.ends[1] > t->key_max) t->key_max = h.ends[1];
+  if (!h.user[kUserOverflow]) return HM_OK;
 
-  cudaMemsetAsync(dflags, 0, 8, s);
-  if (n <= kSmallSort) {
-    small_sort_unique_kernel<<<1, 1024, 0, s>>>(d_keys, d_vals, (int)n, bk, bv, at + n, dflags);
-    note_launch();
-  } else {
-    transform_keys_in(d_keys, uk, n, s);
-    if (radix_sort_positions(uk, idx, uk_alt, idx_alt, n, 0, 64, sort_scratch, s)) {
-      std::swap(uk, uk_alt);
-      std::swap(idx, idx_alt);
-    }
-    last_occurrence_kernel<<<grid_for(n), kThreads, 0, s>>>(uk, n, keep, dflags);
-    exclusive_scan_i32(keep, at, n, scan_scratch, s);
-    compact_batch_kernel<<<grid_for(n), kThreads, 0, s>>>(uk, idx, d_vals, keep, at, n, bk, bv);
-    note_launch(2);
-  }
-  run_start = reinterpret_cast<int64_t *>(idx_alt);
-  int64_t hm_[2] = {0, 0};
-  unsigned hf = 0;
-  cudaMemcpyAsync(&hm_[0], at + n, 8, cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&hf, dflags, 4, cudaMemcpyDeviceToHost, s);
-  cudaError_t e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_err(e);
-  if (hf & 2u) return HM_EMAXKEY;
-  const int64_t m = hm_[0];
-
-  apply_kernel<<<grid_for(m), kThreads, 0, s>>>(t->view(), f, lc, li, flags, bk, bv, m, t->leaf_rows,
-                                                miss, leaf_of);
-  exclusive_scan_i32(miss, at, m, scan_scratch, s);
-  compact_miss_kernel<<<grid_for(m), kThreads, 0, s>>>(bk, bv, leaf_of, miss, at, m, mk, mv, ml);
+  // Some leaf has no room for its new keys: rebalance the subtrees (last-level
+  // nodes) that have room; if one has none, rebuild the tree.
+  auto take = [&](size_t b) { char *r = p; p += b; return r; };
+  int64_t *at = reinterpret_cast<int64_t *>(take(s8));
+  int64_t *mk = reinterpret_cast<int64_t *>(take(s8));
+  int64_t *mv = reinterpret_cast<int64_t *>(take(s8));
+  int32_t *miss = reinterpret_cast<int32_t *>(take(s4));
+  int32_t *ml = reinterpret_cast<int32_t *>(take(s4));
+  int32_t *is_start = reinterpret_cast<int32_t *>(take(s4));
+  int32_t *run_len = reinterpret_cast<int32_t *>(take(s4));
+  int32_t *run_leaf = reinterpret_cast<int32_t *>(take(s4));
+  int32_t *run_parent = reinterpret_cast<int32_t *>(take(s4));
+  int32_t *mark = reinterpret_cast<int32_t *>(p);
+  left_over_kernel<<<grid_for(n), kThreads, 0, s>>>(ep.sk, ep.leaf_of, ep.mask, n, lc, li, t->leaf_rows, miss);
+  exclusive_scan_i32(miss, at, n, ep.scan_scratch, s);
+  compact_miss_kernel<<<grid_for(n), kThreads, 0, s>>>(ep.sk, ep.spos, d_vals, ep.leaf_of, miss, at, n, mk, mv, ml);
   note_launch(2);
-  cudaMemcpyAsync(&hm_[1], at + m, 8, cudaMemcpyDeviceToHost, s);
-  e = cudaStreamSynchronize(s);
+  int64_t nm = 0;
+  cudaError_t e = cudaMemcpyAsync(&nm, at + n, 8, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_err(e);
-  const int64_t nm = hm_[1];
-  if (nm == 0) return HM_OK;
-
-  cudaMemsetAsync(dflags, 0, 4, s);
-  miss_runs_kernel<<<grid_for(nm), kThreads, 0, s>>>(ml, nm, t->leaf_cnt, lc, run_start, run_len,
-                                                      run_leaf, is_start, dflags);
-  note_launch();
-  cudaMemcpyAsync(&hf, dflags, 4, cudaMemcpyDeviceToHost, s);
-  int64_t new_ends[2];
-  cudaMemcpyAsync(&new_ends[0], mk, 8, cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&new_ends[1], mk + nm - 1, 8, cudaMemcpyDeviceToHost, s);
-  e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_err(e);
-
-  // Some leaf overflows: rebalance the subtrees (last-level nodes) that have
-  // room; if one has none, rebuild the tree.
-  int32_t *mark = nullptr, *run_parent = nullptr;
   const Subtree g{t->lvl_start[t->height - 1], t->n_inner, t->n_inner, t->n_leaf};
   const int64_t last_nodes = g.lvl1 - g.lvl0;
-  if (hf & 1u) {
-    run_parent = keep;  // free after the batch compaction; nm <= n entries
-    mark = marks;
-    cudaMemsetAsync(mark, 0, 4 * last_nodes, s);
-    subtree_mark_kernel<<<grid_for(nm), kThreads, 0, s>>>(t->prefix, t->leaf_cnt, t->leaf_base, lc, g, is_start,
-                                                           run_len, run_leaf, ml, nm, run_parent, mark, dflags);
+  miss_runs_kernel<<<grid_for(nm), kThreads, 0, s>>>(ml, nm, run_len, run_leaf, is_start);
+  cudaMemsetAsync(mark, 0, 4 * last_nodes, s);
+  subtree_mark_kernel<<<grid_for(nm), kThreads, 0, s>>>(t->prefix, t->leaf_cnt, t->leaf_base, lc, g, is_start, run_len,
+                                                         run_leaf, ml, nm, run_parent, mark, &ep.ctl->flags);
+  note_launch(2);
+  rc = ep.read(&h, s);
+  if (rc) return rc;
+  if (!(h.flags & 4u)) {
+    const size_t smem = (size_t)t->cfg.fanout * lc * sizeof(longlong2);
+    rc = opt_in_smem((const void *)subtree_rebalance_kernel, 128 * 64 * (int)sizeof(longlong2));  // up to 128 KiB
+    if (rc) return rc;
+    subtree_rebalance_kernel<<<(unsigned)last_nodes, kThreads, smem, s>>>(
+        t->inner, t->prefix, t->leaf_rows, t->leaf_cnt, t->leaf_base, t->cfg.fanout, lc, li, g, mark, mk, mv, ml, nm);
     note_launch();
-    e = cudaMemcpyAsync(&hf, dflags, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    t->shape_version++;  // separators of the last inner level changed
+    e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_err(e);
-  }
-  if (!(hf & 4u)) {
-    // Every touched leaf has room, or its subtree does: merge in place.
-    int64_t blocks = (nm + 7) / 8;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    merge_leaf_kernel<<<(unsigned)blocks, kThreads, 0, s>>>(t->leaf_rows, t->leaf_cnt, lc,
-                                                            li, mk, mv, is_start, run_start, run_len,
-                                                            run_leaf, nm, run_parent, mark);
-    note_launch();
-    if (hf & 1u) {
-      const size_t smem = (size_t)t->cfg.fanout * lc * sizeof(longlong2);
-      rc = opt_in_smem((const void *)subtree_rebalance_kernel, 128 * 64 * (int)sizeof(longlong2));  // up to 128 KiB
-      if (rc) return rc;
-      subtree_rebalance_kernel<<<(unsigned)last_nodes, kThreads, smem, s>>>(
-          t->inner, t->prefix, t->leaf_rows, t->leaf_cnt, t->leaf_base, t->cfg.fanout, lc, li, g, mark, mk, mv, ml,
-          nm);
-      note_launch();
-      t->shape_version++;  // separators of the last inner level changed
-      e = cudaGetLastError();
-      if (e != cudaSuccess) return cuda_err(e);
-    }
-    exclusive_scan_i32(t->leaf_cnt, lbase_tmp, t->n_leaf, scan_scratch, s);
-    cudaMemcpyAsync(t->leaf_base, lbase_tmp, 8 * t->n_leaf, cudaMemcpyDeviceToDevice, s);
+    rescan_leaf_base(t, nullptr, ep.scan_scratch, s);
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_err(e);
     t->n_keys += nm;
-  } else {
-    // Rebuild: contents (already carrying this epoch's in-place updates)
-    // merged with the misses, then a bulk load into a fresh arena.
-    const int64_t n0 = t->n_keys, n1 = n0 + nm;
-    const int64_t tn = std::max<int64_t>(n1, 1);
-    char *tmp = nullptr;
-    e = dev_alloc(reinterpret_cast<void **>(&tmp), 4 * al(8 * tn));
-    if (e != cudaSuccess) return cuda_err(e);
-    int64_t *ek = reinterpret_cast<int64_t *>(tmp);
-    int64_t *ev = reinterpret_cast<int64_t *>(tmp + al(8 * tn));
-    uint64_t *ck = reinterpret_cast<uint64_t *>(tmp + 2 * al(8 * tn));
-    int64_t *cv = reinterpret_cast<int64_t *>(tmp + 3 * al(8 * tn));
-    export_contents(t, ek, ev, s);
-    merge_rank_kernel<<<grid_for(n0), kThreads, 0, s>>>(ek, ev, n0, mk, nm, true, ck, cv);
-    merge_rank_kernel<<<grid_for(nm), kThreads, 0, s>>>(mk, mv, nm, ek, n0, true, ck, cv);
-    note_launch(2);
-    rc = rebuild_from_sorted(t, ck, cv, n1, s);
-    release_after(tmp, s);
-    if (rc) return rc;
+    return HM_OK;
   }
-  if (t->n_keys == nm || new_ends[0] < t->key_min) t->key_min = new_ends[0];
-  if (t->n_keys == nm || new_ends[1] > t->key_max) t->key_max = new_ends[1];
-  return HM_OK;
+  // Rebuild: contents (already carrying the rest of this epoch) merged with
+  // the left-over keys, then a bulk load into a fresh arena.
+  const int64_t n0 = t->n_keys, n1 = n0 + nm;
+  const int64_t tn = std::max<int64_t>(n1, 1);
+  char *tmp = nullptr;
+  e = dev_alloc(reinterpret_cast<void **>(&tmp), 4 * al(8 * tn));
+  if (e != cudaSuccess) return cuda_err(e);
+  int64_t *ek = reinterpret_cast<int64_t *>(tmp);
+  int64_t *ev = reinterpret_cast<int64_t *>(tmp + al(8 * tn));
+  uint64_t *ck = reinterpret_cast<uint64_t *>(tmp + 2 * al(8 * tn));
+  int64_t *cv = reinterpret_cast<int64_t *>(tmp + 3 * al(8 * tn));
+  export_contents(t, ek, ev, s);
+  merge_rank_kernel<<<grid_for(n0), kThreads, 0, s>>>(ek, ev, n0, mk, nm, true, ck, cv);
+  merge_rank_kernel<<<grid_for(nm), kThreads, 0, s>>>(mk, mv, nm, ek, n0, true, ck, cv);
+  note_launch(2);
+  rc = rebuild_from_sorted(t, ck, cv, n1, s);
+  release_after(tmp, s);
+  return rc;
 }
 
 // One epoch of deletes (no counterpart in the reference, whose
 // BPlusTree::remove is an empty stub, open-harmonia/src/bpt.cpp:771-773):
-// sort the batch and drop repeats, mark each stored key's slot, compact the
-// touched leaves in place and rescan leaf_base.  Separators stay valid (the
-// remaining keys of leaf j still lie between its separators), so the inner
-// levels are untouched.  A leaf left empty would break the invariant that
-// every leaf's first key is a key of the leaf (the bucket join searches
-// leaves by first key), so such an epoch ends in a rebuild of the remaining
-// contents instead.
-int delete_epoch(hm_tree *t, const int64_t *d_keys, int64_t n, int64_t *removed_out, cudaStream_t s) {
+// sort the batch, mark each stored key's slot, squeeze the touched leaves in
+// place and rescan leaf_base.  Separators stay valid (the remaining keys of
+// leaf j still lie between its separators), so the inner levels are
+// untouched.  A leaf left empty would break the invariant that every leaf's
+// first key is a key of the leaf (the bucket join searches leaves by first
+// key), so such an epoch ends in a rebuild of the remaining contents instead.
+int delete_epoch(hm_tree *t, const int64_t *d_keys, int64_t n, int64_t *removed_out, unsigned *err, cudaStream_t s) {
   if (removed_out) *removed_out = 0;
   if (n <= 0) return HM_OK;
   if (n > kMaxEpochKeys) return HM_ETOOLARGE;
-  const int lc = t->cfg.leaf_cap, li = t->leaf_index, f = t->cfg.fanout;
-  const size_t s8 = al(8 * (n + 1)), s4 = al(4 * (n + 1));
-  const int64_t scan_n = std::max<int64_t>(n, t->n_leaf) + 1;
-  const size_t lb8 = al(8 * (t->n_leaf + 1));
-  size_t need = 6 * s8 + 2 * s4 + lb8 + al((int64_t)radix_scratch_bytes(n)) +
-                al((int64_t)scan_scratch_bytes(scan_n)) + 256;
   ScratchLease lease(t, s);
-  int rc = lease.acquire(need);
+  int rc = lease.acquire(Epoch::bytes(t, n));
   if (rc) return rc;
-  char *p = static_cast<char *>(lease.ptr());
-  auto take8 = [&](void) { char *r = p; p += s8; return r; };
-  auto take4 = [&](void) { char *r = p; p += s4; return r; };
-  uint64_t *uk = reinterpret_cast<uint64_t *>(take8());
-  uint64_t *uk_alt = reinterpret_cast<uint64_t *>(take8());
-  int32_t *idx = reinterpret_cast<int32_t *>(take8());
-  int32_t *idx_alt = reinterpret_cast<int32_t *>(take8());
-  int64_t *at = reinterpret_cast<int64_t *>(take8());
-  int64_t *bk = reinterpret_cast<int64_t *>(take8());
-  int32_t *keep = reinterpret_cast<int32_t *>(take4());
-  int32_t *route = reinterpret_cast<int32_t *>(take4());
-  void *sort_scratch = p;
-  p += al((int64_t)radix_scratch_bytes(n));
-  int64_t *lbase_tmp = reinterpret_cast<int64_t *>(p);  // n_leaf + 1 entries
-  p += lb8;
-  void *scan_scratch = p;
-  p += al((int64_t)scan_scratch_bytes(scan_n));
-  unsigned long long *dremoved = reinterpret_cast<unsigned long long *>(p);
-  unsigned *dflags = reinterpret_cast<unsigned *>(p + 8);
-
-  cudaMemsetAsync(p, 0, 16, s);
-  if (n <= kSmallSort) {
-    small_sort_unique_kernel<<<1, 1024, 0, s>>>(d_keys, nullptr, (int)n, bk, nullptr, at + n, dflags);
-    note_launch();
-  } else {
-    transform_keys_in(d_keys, uk, n, s);
-    if (radix_sort_positions(uk, idx, uk_alt, idx_alt, n, 0, 64, sort_scratch, s)) std::swap(uk, uk_alt);
-    last_occurrence_kernel<<<grid_for(n), kThreads, 0, s>>>(uk, n, keep, dflags);
-    exclusive_scan_i32(keep, at, n, scan_scratch, s);
-    compact_keys_kernel<<<grid_for(n), kThreads, 0, s>>>(uk, keep, at, n, bk);
-    note_launch(2);
-  }
-  int64_t m = 0;
-  cudaMemcpyAsync(&m, at + n, 8, cudaMemcpyDeviceToHost, s);
-  cudaError_t e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_err(e);
-
-  delete_mark_kernel<<<grid_for(m), kThreads, 0, s>>>(t->view(), f, lc, li, bk, m, t->leaf_rows, route);
-  cudaMemsetAsync(dflags, 0, 4, s);  // the Max_Key bit of the dedup pass is not an error here
-  delete_compact_kernel<<<grid_for(m), kThreads, 0, s>>>(t->leaf_rows, t->leaf_cnt, lc, li, route, m, dremoved,
-                                                          dflags);
-  note_launch(2);
-  unsigned long long removed = 0;
-  unsigned hf = 0;
-  cudaMemcpyAsync(&removed, dremoved, 8, cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&hf, dflags, 4, cudaMemcpyDeviceToHost, s);
-  e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_err(e);
-  if (removed_out) *removed_out = (int64_t)removed;
-  if (removed == 0) return HM_OK;
-  exclusive_scan_i32(t->leaf_cnt, lbase_tmp, t->n_leaf, scan_scratch, s);
-  cudaMemcpyAsync(t->leaf_base, lbase_tmp, 8 * t->n_leaf, cudaMemcpyDeviceToDevice, s);
-  e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_err(e);
-  t->n_keys -= (int64_t)removed;
-  if (!(hf & 1u)) return HM_OK;
+  Epoch ep;
+  ep.place(t, n, static_cast<char *>(lease.ptr()));
+  bsort::Ctl h{};
+  rc = ep.run(t, d_keys, nullptr, 0, true, &h, s);
+  if (rc) return rc;
+  *err = (unsigned)h.user[kUserErr];
+  const int64_t removed = (int64_t)h.user[kUserChanged];
+  if (removed_out) *removed_out = removed;
+  t->n_keys -= removed;
+  if (!h.user[kUserEmpty]) return HM_OK;
   // a leaf emptied: rebuild from the remaining contents
   const int64_t n1 = t->n_keys, tn = std::max<int64_t>(n1, 1);
   char *tmp = nullptr;
-  e = dev_alloc(reinterpret_cast<void **>(&tmp), 3 * al(8 * tn));
+  cudaError_t e = dev_alloc(reinterpret_cast<void **>(&tmp), 3 * al(8 * tn));
   if (e != cudaSuccess) return cuda_err(e);
   int64_t *ek = reinterpret_cast<int64_t *>(tmp);
   int64_t *ev = reinterpret_cast<int64_t *>(tmp + al(8 * tn));
