@@ -1062,7 +1062,7 @@ int range_impl(hm_tree *t, const int64_t *start, const int32_t *len, const int64
   if (!okeys || !ovals) return HM_EINVAL;
   const bool dev_rec = is_device_ptr(okeys) && is_device_ptr(ovals);
   if (dev_rec) {
-    rc = range_copy_out(t, fl, fs, d_off, n, okeys, ovals, s);
+    rc = range_copy_out(t, fl, fs, d_off, n, (int64_t)cap, okeys, ovals, s);
     prof_end(t, kStageRange, tok, s);
     if (rc) return rc;
     return hm_sync(t, hs);
@@ -1073,7 +1073,7 @@ int range_impl(hm_tree *t, const int64_t *start, const int32_t *len, const int64
   e = cudaMallocAsync(reinterpret_cast<void **>(&tk), 2 * (size_t)align_up(tot * 8, 256), s);
   if (e != cudaSuccess) return cuda_err(e);
   int64_t *tv = reinterpret_cast<int64_t *>(reinterpret_cast<char *>(tk) + align_up(tot * 8, 256));
-  rc = range_copy_out(t, fl, fs, d_off, n, tk, tv, s);
+  rc = range_copy_out(t, fl, fs, d_off, n, tot, tk, tv, s);
   prof_end(t, kStageRange, tok, s);
   if (rc == HM_OK) {
     e = cudaMemcpyAsync(okeys, tk, tot * 8, cudaMemcpyDeviceToHost, s);

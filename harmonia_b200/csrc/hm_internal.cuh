@@ -381,7 +381,8 @@ size_t range_scratch_bytes(int64_t n);
 int range_locate(const hm_tree *t, const int64_t *start, const int32_t *len, const int64_t *end, int64_t n,
                  int32_t *first_leaf, int32_t *first_slot, int64_t *count, cudaStream_t s);
 int range_copy_out(const hm_tree *t, const int32_t *first_leaf, const int32_t *first_slot,
-                   const int64_t *offsets, int64_t n, int64_t *okeys, int64_t *ovals, cudaStream_t s);
+                   const int64_t *offsets, int64_t n, int64_t cap, int64_t *okeys, int64_t *ovals,
+                   cudaStream_t s);  // nothing if offsets[n] > cap
 
 // ---- upsert (upsert.cu) ----
 // Both return when done; *err: the tree's error word during the epoch.

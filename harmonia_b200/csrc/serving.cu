@@ -390,7 +390,7 @@ int launch_ranges(hm_server *sv, Slot &sl) {
   rc = range_locate(t, ds, dl, nullptr, n, fl, fs, cnt, sl.s);
   if (rc) return rc;
   exclusive_scan_i64(cnt, off, n, scan, sl.s);
-  rc = range_copy_out(t, fl, fs, off, n, ok, ov, sl.s);
+  rc = range_copy_out(t, fl, fs, off, n, INT64_MAX, ok, ov, sl.s);
   if (rc) return rc;
   e = cudaEventRecord(sl.kdone, sl.s);
   if (e != cudaSuccess) return cuda_err(e);
