@@ -27,10 +27,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
                : "memory");
 }
 
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
+__device__ __forceinline__ void bulk_g2s(unsigned dst, const void *src, unsigned bytes, uint64_t *bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_addr(dst)),
+          "r"(dst),
       "l"(src), "r"(bytes), "r"(smem_addr(bar))
       : "memory");
 }
@@ -60,12 +60,12 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 
 // 2-D tiled TMA load of one box of the tensor map at tmap (the address of a
 // __grid_constant__ kernel parameter) at element coordinates (x, y) into
-// shared memory; completion is counted on bar.  No multicast.  x times the
+// shared memory at address dst; completion is counted on bar.  No multicast.  x times the
 // element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, int x, int y, uint64_t *bar) {
+__device__ __forceinline__ void tma_load_2d(unsigned dst, const void *tmap, int x, int y, uint64_t *bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-      "[%4];" ::"r"(smem_addr(dst)),
+      "[%4];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(smem_addr(bar))
       : "memory");
 }

@@ -8,8 +8,7 @@
 
 #include <algorithm>
 #include <mutex>
-#include <set>
-#include <tuple>
+#include <map>
 #include <unordered_map>
 #include <vector>
 #include <atomic>
@@ -515,7 +514,7 @@ int run_planned_search(hm_tree *t, const SearchPlan &p, const int64_t *d_q, int6
   int64_t *res = reinterpret_cast<int64_t *>(b + align_up(n * 8, 256));
   char *ps = b + 2 * align_up(n * 8, 256);
   char *js = ps + partition_scratch_bytes(n, p.bits, true, p.batches);
-  const int64_t *bstart = nullptr;
+  const uint32_t *bstart = nullptr;
   if (p.placed) {  // the join places results in first-pass order: one inverse pass
     int32_t *place = reinterpret_cast<int32_t *>(js + join_scratch_bytes(n, p.bits));
     int tok = prof_begin(t, s);
@@ -553,16 +552,17 @@ int run_planned_search(hm_tree *t, const SearchPlan &p, const int64_t *d_q, int6
 
 int opt_in_smem(const void *fn, int bytes) {
   static std::mutex mu;
-  static std::set<std::tuple<const void *, int, int>> done;
+  static std::map<std::pair<const void *, int>, int> done;  // the largest size so far: never lowered
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_err(e);
   std::lock_guard<std::mutex> lk(mu);
-  if (done.count({fn, dev, bytes})) return HM_OK;
+  int &most = done[{fn, dev}];
+  if (bytes <= most) return HM_OK;
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return cuda_err(e);
-  done.insert({fn, dev, bytes});
+  most = bytes;
   return HM_OK;
 }
 

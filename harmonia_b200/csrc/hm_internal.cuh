@@ -344,22 +344,22 @@ struct BatchView {
 // written to res1[place[i]] are in first-pass order, which
 // unpermute_first_pass takes back to the input order.
 int partition_queries_placed(const hm_tree *t, const int64_t *q, int64_t n, int bits, int64_t *q_out,
-                             int32_t *place, void *scratch, cudaStream_t s, const int64_t **bucket_start,
+                             int32_t *place, void *scratch, cudaStream_t s, const uint32_t **bucket_start,
                              const BatchView *bv = nullptr);
 int unpermute_first_pass(int64_t n, int bits, const int64_t *res1, int64_t *out, void *scratch, cudaStream_t s,
                          const BatchView *bv = nullptr);
 
-// offsets: the partition keeps chunk offsets in the scratch for
+// offsets: the partition keeps tile offsets in the scratch for
 // unpermute_results (pos_out == nullptr); else it writes input positions.
 size_t partition_scratch_bytes(int64_t n, int bits, bool offsets, int batches = 1);  // batches: of a batch set
 // Groups queries by the top `bits` bits of their key (relative to the tree's
 // key range); *bucket_start (if given) receives a device pointer, inside the
 // scratch, to the 2^bits + 1 bucket starts.  pos_out: original position of
-// each grouped query, or nullptr for the offset mode.
+// each grouped query (bits <= 8), or nullptr for the offset mode.
 // With bv, the queries are read from the batch set instead of q.
 int partition_queries(const hm_tree *t, const int64_t *q, int64_t n, int bits,
                       int64_t *q_out, int32_t *pos_out, void *scratch, cudaStream_t s,
-                      const int64_t **bucket_start = nullptr, const BatchView *bv = nullptr);
+                      const uint32_t **bucket_start = nullptr, const BatchView *bv = nullptr);
 // Offset mode: out[i] = result of input query i, given the results in grouped
 // order (res_sorted, clobbered) and the scratch of the matching partition.
 // With bv, the results go to the batch set's outputs instead of out.
@@ -404,12 +404,11 @@ bool join_fits(const hm_tree *t);  // the join supports this leaf size and its b
 size_t join_scratch_bytes(int64_t n, int bits);
 // place: nullptr = results in grouped order (out[i] for grouped query i);
 // else out[place[i]].
-int launch_join(const hm_tree *t, const int64_t *qs, const int64_t *bstart, int bits, int64_t n, int64_t *out,
+int launch_join(const hm_tree *t, const int64_t *qs, const uint32_t *bstart, int bits, int64_t n, int64_t *out,
                 void *scratch, cudaStream_t s, const int32_t *place = nullptr);
 
-// Opts kernel fn in to `bytes` of dynamic shared memory (and the largest
-// shared-memory carveout) on the current device; once per device, kernel and
-// size, from any thread.
+// Opts kernel fn in to at least `bytes` of dynamic shared memory (and the
+// largest shared-memory carveout) on the current device, from any thread.
 int opt_in_smem(const void *fn, int bytes);
 
 // ---- search plan (harmonia.cu) ----

@@ -5,15 +5,14 @@
 // contiguous run and the bucket's keys lie in a contiguous range of leaves.
 // Instead of one descent per query (search.cu), a CTA takes a run of one
 // bucket, copies the bucket's leaf records (keys and values, 256 B per
-// 16-key leaf) from HBM into shared memory in order (2-D tiled TMA loads for
-// 16-key leaves, per-thread cp.async otherwise), and
-// answers every query of the run from shared memory: a binary search over the
-// leaves' first keys (or, for batches of many queries per bucket, a 64-slot
-// directory of them built once per run) picks the leaf, a binary search of
-// its keys the slot.  The leaf range of each bucket comes from one descent per
-// bucket boundary (a separate kernel, one thread per boundary; kept per tree
-// shape between calls).  Leaves are read once per run
-// and sequentially, so the DRAM traffic of a batch with more queries than
+// 16-key leaf) from HBM into shared memory in order, and answers every query of
+// the run from there.  16-key leaves are staged by TMA and searched through
+// 31-bit images of their first keys (join_tma_kernel); 64-key leaves, and
+// batches of many queries per bucket, which first build a 64-slot directory of
+// the bucket, by per-thread cp.async (join_kernel).  The leaf range of each
+// bucket comes from one descent per bucket boundary (a separate kernel, one
+// thread per boundary; kept per tree shape between calls).  Leaves are read once
+// per run and sequentially, so the DRAM traffic of a batch with more queries than
 // leaves falls from a random 160 B per query to the size of the touched leaf
 // region.  A bucket whose leaves do not fit shared memory (very skewed keys)
 // falls back to a scalar descent per query.  For batches up to 2^25 queries
@@ -44,16 +43,13 @@ constexpr int kThreads = 256;
 #endif
 constexpr int kPerThread = HM_JOIN_PER_THREAD;
 constexpr int kRun = kThreads * kPerThread;  // queries a CTA answers per step
-#ifndef HM_JOIN_ITEM_RUNS
-#define HM_JOIN_ITEM_RUNS 64
-#endif
-// Steps of one work item: a bucket with more queries is cut into items of
-// kItemMax (hot buckets of a skewed batch); each item stages its bucket's
-// leaves once, so larger items re-read a hot bucket's leaves less often
-// (measured on the 217 M-query batch set, half Zipf: join 1.60 ms with
-// 4096-query items, 1.48 with 8192, 1.44 with 16384).
-constexpr int kItemRuns = HM_JOIN_ITEM_RUNS;
-constexpr int kItemMax = kRun * kItemRuns;  // queries per work item, at most
+// Queries per work item of the cp.async join, at most: a bucket with more is
+// cut into items (hot buckets of a skewed batch), each of which stages the
+// bucket's leaves.  Small items keep the CTAs evenly loaded when a few keys
+// draw many queries, large ones stage less: a sixteenth of an SM's share of the
+// batch, between the two bounds (6 M Zipf queries on 64-key leaves: 218 us with
+// items of 16384, 135 with 2560, 148 with 5120, 142 with 634).
+constexpr int kItemMin = 1024, kItemMax = 16384;
 static_assert(kItemMax < 65536, "an item's query count is kept in 16 bits");
 #ifndef HM_JOIN_STAGES
 #define HM_JOIN_STAGES 2  // shared-memory ring of the join kernel
@@ -72,28 +68,23 @@ constexpr int kStageMax = (216 / kStages) * 1024;  // shared memory of one stage
 #endif
 static_assert(HM_JOIN_MAX_BITS <= 16, "a bucket number is kept in 16 bits");
 
-// A work item: at most kItemMax queries of one bucket, grouped queries
+// A work item: some queries of one bucket, grouped queries
 // [qa, qa + len), and the bucket's leaves [l0, l0 + nl); the leaves are
 // staged once for all of them.
 struct __align__(16) Item {
   int32_t qa, l0, b;  // first query, first leaf, bucket
-  uint32_t len_nl;    // queries (at most kItemMax) << 16 | leaves (capped at 65535)
+  uint32_t len_nl;    // queries << 16 | leaves (capped at 65535)
   __host__ __device__ int len() const { return (int)(len_nl >> 16); }
   __host__ __device__ int nl() const { return (int)(len_nl & 0xffffu); }
 };
 
-// Per bucket b in [0, nb]: cnt[b] = its work items (0 for b = nb) and, with
-// want_leafb, leafb[b] = leaf holding the smallest key of bucket b (bucket
-// b's keys lie in leaves [leafb[b], leafb[b+1]]).  leafb depends only on the
+// leafb[b], b in [0, nb] = leaf holding the smallest key of bucket b (bucket
+// b's keys lie in leaves [leafb[b], leafb[b+1]]).  It depends only on the
 // inner nodes, the key range and the bucket bits, so the launcher keeps it
 // per tree shape and skips the descents while that holds.
-__global__ void bucket_prep_kernel(DevTree t, int f, int64_t lo, int shift, int nb,
-                                   const int64_t *__restrict__ bstart, int32_t *__restrict__ leafb,
-                                   int32_t *__restrict__ cnt, bool want_leafb) {
+__global__ void bucket_bounds_kernel(DevTree t, int f, int64_t lo, int shift, int nb, int32_t *__restrict__ leafb) {
   pdl_enter();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x) {
-    if (cnt) cnt[b] = b < nb ? (int32_t)((bstart[b + 1] - bstart[b] + kItemMax - 1) / kItemMax) : 0;
-    if (!want_leafb) continue;
     if (b == 0) {
       leafb[0] = 0;
       continue;
@@ -111,26 +102,50 @@ __global__ void bucket_prep_kernel(DevTree t, int f, int64_t lo, int shift, int 
   }
 }
 
-// Bucket b's items start at first[b] (exclusive scan of cnt).
-__global__ void expand_items_kernel(int nb, const int64_t *__restrict__ bstart, const int32_t *__restrict__ leafb,
-                                    const int32_t *__restrict__ cnt, const int64_t *__restrict__ first,
-                                    Item *__restrict__ items) {
+// The work items in bucket order and their number: CTA c owns buckets
+// [1024 c, 1024 c + 1024) and counts the items of those before them itself (at
+// most 64 loads a thread).
+constexpr int kItemThreads = 1024;
+
+__global__ void __launch_bounds__(kItemThreads) items_kernel(int nb, uint32_t item_max,
+                                                             const uint32_t *__restrict__ bstart,
+                                                             const int32_t *__restrict__ leafb,
+                                                             Item *__restrict__ items, int64_t *__restrict__ n_items) {
   pdl_enter();
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-    const int c = cnt[b];
-    if (c == 0) continue;
-    const int64_t s = bstart[b], e = bstart[b + 1];
-    const int32_t l0 = leafb[b], nl = leafb[b + 1] - l0 + 1;
-    int64_t o = first[b];
-    for (int r = 0; r < c; r++) {
-      Item it;
-      it.qa = (int32_t)(s + (int64_t)r * kItemMax);
-      const int32_t len = (int32_t)min((int64_t)kItemMax, e - (s + (int64_t)r * kItemMax));
-      it.l0 = l0;
-      it.b = b;
-      it.len_nl = (uint32_t)len << 16 | (uint32_t)min(nl, 65535);  // a capped count is never staged
-      items[o + r] = it;
-    }
+  __shared__ uint32_t wsum[32], bsum[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int first = blockIdx.x * kItemThreads;
+  auto items_of = [&](int b) { return (bstart[b + 1] - bstart[b] + item_max - 1) / item_max; };
+  uint32_t before = 0;
+  for (int b = tid; b < first; b += kItemThreads) before += items_of(b);
+  const int b = first + tid;
+  const uint32_t mine = b < nb ? items_of(b) : 0;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  uint32_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) wsum[warp] = incl;
+  if (lane == 0) bsum[warp] = before;
+  __syncthreads();
+  uint32_t at = incl - mine;
+  for (int w = 0; w < 32; w++) at += bsum[w];
+  for (int w = 0; w < warp; w++) at += wsum[w];
+  if (b == nb - 1) *n_items = at + mine;
+  if (mine == 0) return;
+  const uint32_t s = bstart[b], e = bstart[b + 1];
+  const int32_t l0 = leafb[b], nl = leafb[b + 1] - l0 + 1;
+  for (uint32_t r = 0; r < mine; r++) {
+    const uint32_t qa = s + r * item_max;
+    Item it;
+    it.qa = (int32_t)qa;
+    it.l0 = l0;
+    it.b = b;
+    it.len_nl = min(item_max, e - qa) << 16 | (uint32_t)min(nl, 65535);  // a capped count is never staged
+    items[at + r] = it;
   }
 }
 
@@ -162,28 +177,6 @@ struct Stage {
   __device__ __forceinline__ int64_t first(int m) const { return kp[m * (LC + 1)]; }
   __device__ __forceinline__ int64_t key(int m, int c) const { return kp[m * (LC + 1) + c]; }
   __device__ __forceinline__ int64_t val(int m, int c) const { return vp[m * LC + c]; }
-};
-
-// A stage filled by 2-D tiled TMA loads of 16-key leaf records (LC = 16):
-// the keys of leaf m in 128-B row m of the key block, the values in row m of
-// the value block, both in the TMA's 128-B swizzle (16-B chunk j of row m at
-// chunk j ^ (m mod 8); the blocks start on 1024-B boundaries), and the
-// leaves' first keys copied densely once the loads land (the binary search
-// over them then reads consecutive words).
-struct StageTma {
-  const unsigned char *kb, *vb;
-  const int64_t *firsts;
-  __device__ StageTma(const unsigned char *k, const unsigned char *v, const int64_t *f) : kb(k), vb(v), firsts(f) {}
-  __device__ __forceinline__ static int off(int m, int c) {
-    return m * 128 + ((((c >> 1) ^ m) & 7) << 4) + ((c & 1) << 3);
-  }
-  __device__ __forceinline__ int64_t first(int m) const { return firsts[m]; }
-  __device__ __forceinline__ int64_t key(int m, int c) const {
-    return *reinterpret_cast<const int64_t *>(kb + off(m, c));
-  }
-  __device__ __forceinline__ int64_t val(int m, int c) const {
-    return *reinterpret_cast<const int64_t *>(vb + off(m, c));
-  }
 };
 
 // Asynchronous copy of an item's leaf records into a stage (nothing when the
@@ -409,120 +402,245 @@ __global__ void __launch_bounds__(kThreads, HM_JOIN_MINB) join_kernel(DevTree t,
   cp_async_wait_all();
 }
 
-// The join for 16-key leaf records with the stages filled by the tensor
-// memory accelerator: one thread issues, per item, 2-D tiled loads of 8
-// records at a time (one box for their keys, one for their values, 1 KiB
-// each, 128-B swizzle) that complete on the stage's mbarrier; the other
-// threads do no address work for the staging.  An item's last box may bring
-// up to 7 records past its range (the next bucket's leaves, or zeros past the
-// last leaf), which are never searched.  Every wait is bounded: on a timeout
-// the CTA records HM_ETIMEOUT in err, waits (bounded) for the loads it issued
-// and returns.
-template <bool DIR, bool PLACED>
-__global__ void __launch_bounds__(kThreads, HM_JOIN_MINB) join_tma_kernel(
+// The join for 16-key leaf records: a producer warp fills a ring of stages, the
+// other warps look up.  An item's stage gets, all counted on its mbarrier, the
+// leaf records by 2-D tiled TMA loads of 8 records at a time (one box for
+// their keys, one for their values, 1 KiB each, 128-B swizzle: 16-B chunk j of
+// row m lies at chunk j ^ (m mod 8); a box per producer lane), the item's first
+// kJoinStep queries and their places by two bulk copies (from the 16-byte
+// boundary below them), and its descriptor.  The last box may bring up to 7
+// records past the item's range (the next bucket's leaves, or zeros past the
+// last leaf), which are never searched.
+//
+// What an item costs is latency, so nothing of it is left to a load by the
+// threads that wait for it, and the lookups are kept short: the leaf is found
+// by a binary search over 31-bit images of the leaves' first keys (their offset
+// from the bucket's lowest key, its top 31 bits; padded, so no step checks a
+// bound), the slot by four probes of the leaf's keys whose swizzled address is
+// one exclusive-or.  Two first keys with one image make the search end on a
+// leaf past the key's, seen by its first key being above the key, and step
+// back.  kJoinStep covers a bucket of 256 queries and four standard deviations.  An item takes one CTA barrier: past it every thread
+// has left the item before, whose stage is then filled again.
+// 2^24 queries on 2^26 keys (1.41 GB of records, queries, places and results):
+// 241 us, 5.9 TB/s, 0.90 of the measured copy rate.  Before, with one thread
+// issuing the loads between its lookups, 64-bit binary searches and one query
+// a thread: 320 us; the producer warp took it to 288, two queries a thread and
+// the fixed step count to 241 (one query a thread: 252).
+//
+// Every wait is bounded: on a timeout the CTA records HM_ETIMEOUT in err, waits
+// (bounded) for the loads it issued and returns.
+constexpr int kJoinThreads = 160;            // that look up
+constexpr int kJoinQueries = 2;              // of a thread at a time
+constexpr int kJoinStep = kJoinThreads * kJoinQueries;
+constexpr int kJoinCtas = 4;                 // resident on an SM
+constexpr uint32_t kImageMax = 0x7fffffffu;  // of a key in the bucket
+constexpr uint32_t kQueryBytes = (kJoinStep + 2) * 8, kPlaceBytes = (kJoinStep + 4) * 4;
+constexpr uint32_t kItemBytes = (kQueryBytes + kPlaceBytes + 16 + 127) / 128 * 128;  // beside the records
+static_assert(kQueryBytes % 16 == 0 && kPlaceBytes % 16 == 0, "bulk copies of whole 16-byte words");
+
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ int64_t lds64(uint32_t a) {
+  int64_t v;
+  asm volatile("ld.shared.s64 %0, [%1];" : "=l"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ Item lds_item(uint32_t a) {
+  Item i;
+  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(i.qa), "=r"(i.l0), "=r"(i.b), "=r"(*reinterpret_cast<int *>(&i.len_nl))
+               : "r"(a)
+               : "memory");
+  return i;
+}
+__device__ __forceinline__ void sts_item(uint32_t a, const Item &i) {
+  asm volatile("st.shared.v4.s32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(i.qa), "r"(i.l0), "r"(i.b), "r"((int)i.len_nl)
+               : "memory");
+}
+
+// Stages of the ring for a span of 2^steps leaves: three of up to 64 leaves or
+// two of more, so that four CTAs share an SM.
+__host__ __device__ constexpr int tma_stages(int steps) { return steps <= 6 ? 3 : 2; }
+
+template <bool PLACED, int STEPS>
+__global__ void __launch_bounds__(kJoinThreads + 32, kJoinCtas) join_tma_kernel(
     const __grid_constant__ CUtensorMap tmap, DevTree t, int f, const Item *__restrict__ items,
     const int64_t *__restrict__ nitems, const int64_t *__restrict__ qs, const int32_t *__restrict__ place,
     int64_t *__restrict__ out, int ml, uint64_t key_lo_u, int shift, unsigned *err) {
-  constexpr int LC = 16;
+  constexpr int LC = 16, STAGES = tma_stages(STEPS);
   pdl_enter();
-  static_assert(kStages >= 2, "a ring of at least two stages");
   extern __shared__ __align__(16) unsigned char dyn[];
-  __shared__ __align__(8) uint64_t bars[kStages];
-  __shared__ int32_t dir[DIR ? kDir + 1 : 1];
-  const int64_t n_items = *nitems;
-  const int64_t g = gridDim.x;
-  int64_t it = blockIdx.x;
+  __shared__ __align__(8) uint64_t bars[STAGES];
+  const int n_items = (int)*nitems, g = (int)gridDim.x, tid = threadIdx.x, lane = tid & 31;
+  int it = blockIdx.x;
   if (it >= n_items) return;
   const int rb = (ml + 7) & ~7;  // rows of a stage's key block (and value block)
-  const int block = rb * 128;
-  unsigned char *base = dyn + ((1024u - (smem_addr(dyn) & 1023u)) & 1023u);  // 1024-B aligned
-  int64_t *firsts = reinterpret_cast<int64_t *>(base + (size_t)kStages * 2 * block);  // [kStages][rb]
-  if (threadIdx.x == 0) {
-    for (int x = 0; x < kStages; x++) mbar_init(&bars[x], 1);
+  const uint32_t block = rb * 128;
+  const uint32_t base = (smem_addr(dyn) + 1023u) & ~1023u;  // the swizzle's period; [stage][keys, values]
+  const uint32_t rest = base + STAGES * 2 * block;      // [stage] queries, places, descriptor
+  const uint32_t images = rest + STAGES * kItemBytes;   // [2][SPAN]
+  constexpr int SPAN = 1 << STEPS;
+  if (tid == 0) {
+    for (int x = 0; x < STAGES; x++) mbar_init(&bars[x], 1);
     fence_mbar_init();
   }
   __syncthreads();
-  // thread 0: the loads of item `itm` into stage x (none for an item that is
-  // not staged: the arrival alone completes the phase)
-  auto issue = [&](const Item &itm, int x) {
-    const bool stg = itm.nl() >= 1 && itm.nl() <= ml;
-    const int boxes = stg ? (itm.nl() + 7) >> 3 : 0;
-    fence_proxy_async_smem();  // the stage's earlier reads come before these writes
-    mbar_expect_tx(&bars[x], (unsigned)boxes * 2048u);
-    unsigned char *kb = base + (size_t)x * 2 * block;
-    for (int b = 0; b < boxes; b++) {
-      tma_load_2d(kb + b * 1024, &tmap, 0, itm.l0 + 8 * b, &bars[x]);
-      tma_load_2d(kb + block + b * 1024, &tmap, 16, itm.l0 + 8 * b, &bars[x]);
+  const int ishift = max(0, shift - 31);
+  const bool producer = tid >= kJoinThreads;
+  // The producer warp: fills stage x with an item (past the last one only a
+  // descriptor of no queries and the arrival).
+  Item mine{0, 0, 0, 0};  // descriptor of this CTA's item number (fetched & ~31) + lane
+  int fetched = 0;
+  auto fill = [&](int x) {
+    if ((fetched & 31) == 0) {
+      const int64_t at = it + (int64_t)(fetched + lane) * g;
+      mine = at < n_items ? items[at] : Item{0, 0, 0, 0};
     }
+    Item itm;
+    itm.qa = __shfl_sync(0xffffffffu, mine.qa, fetched & 31);
+    itm.l0 = __shfl_sync(0xffffffffu, mine.l0, fetched & 31);
+    itm.b = __shfl_sync(0xffffffffu, mine.b, fetched & 31);
+    itm.len_nl = __shfl_sync(0xffffffffu, mine.len_nl, fetched & 31);
+    fetched++;
+    const int boxes = itm.nl() >= 1 && itm.nl() <= ml ? 2 * ((itm.nl() + 7) >> 3) : 0;
+    const int len = min(itm.len(), kJoinStep);
+    // whole 16-byte words around the queries and the places (both buffers end on 256 bytes)
+    const uint32_t qb = len ? ((uint32_t)(len + (itm.qa & 1) + 1) & ~1u) * 8 : 0;
+    const uint32_t pb = PLACED && len ? ((uint32_t)(len + (itm.qa & 3) + 3) & ~3u) * 4 : 0;
+    const uint32_t r = rest + x * kItemBytes;
+    fence_proxy_async_smem();  // the stage's earlier reads come before these writes
+    if (lane == 0) {
+      sts_item(r + kQueryBytes + kPlaceBytes, itm);
+      mbar_expect_tx(&bars[x], (unsigned)boxes * 1024u + qb + pb);
+      if (qb) bulk_g2s(r, qs + (itm.qa & ~1), qb, &bars[x]);
+      if (pb) bulk_g2s(r + kQueryBytes, place + (itm.qa & ~3), pb, &bars[x]);
+    }
+    __syncwarp();
+    for (int b = lane; b < boxes; b += 32)
+      tma_load_2d(base + x * 2 * block + (b & 1) * block + (b >> 1) * 1024, &tmap, (b & 1) * 16, itm.l0 + 8 * (b >> 1),
+                  &bars[x]);
   };
-  const Item none{0, 0, 0, 0};
-  const int dshift = shift > kDirBits ? shift - kDirBits : 0;
-  Item d[kStages];  // items it, it + g, ..., it + (kStages - 1) g
-#pragma unroll
-  for (int x = 0; x < kStages; x++) d[x] = it + x * g < n_items ? items[it + x * g] : none;
-  if (threadIdx.x == 0)
-    for (int x = 0; x < kStages - 1; x++) issue(d[x], x);
-  unsigned phase = 0;  // bit x: parity of stage x's next phase
-  unsigned pending = (1u << (kStages - 1)) - 1;  // bit x: stage x has loads issued and not waited for
-  int64_t q[kPerThread];
-  int32_t qo[kPerThread];
-#pragma unroll
-  for (int j = 0; j < kPerThread; j++) {
-    const int r = j * kThreads + threadIdx.x;
-    const bool in = r < d[0].len();
-    q[j] = in ? __ldg(qs + d[0].qa + r) : 0;
-    qo[j] = PLACED ? (in ? __ldg(place + d[0].qa + r) : 0) : d[0].qa + r;
-  }
-  int cur_stage = 0;
-  for (; it < n_items; it += g) {
-    const int fill = cur_stage == 0 ? kStages - 1 : cur_stage - 1;  // (cur + kStages - 1) % kStages
-    if (threadIdx.x == 0) issue(d[kStages - 1], fill);
-    pending |= 1u << fill;
-    const Item dn = it + kStages * g < n_items ? items[it + kStages * g] : none;
-    const bool ok = mbar_wait_bounded(&bars[cur_stage], (phase >> cur_stage) & 1u, t.wait_polls);
-    phase ^= 1u << cur_stage;
-    pending &= ~(1u << cur_stage);
+  if (producer)
+    for (int x = 0; x < STAGES - 1; x++) fill(x);
+  const int mine_n = (n_items - it + g - 1) / g;  // this CTA's items
+  unsigned phase = 0;                             // bit x: parity of stage x's next phase
+  for (int i = 0, st = 0; i < mine_n; i++, st = st == STAGES - 1 ? 0 : st + 1) {
+    const bool ok = producer || mbar_wait_bounded(&bars[st], (phase >> st) & 1u, t.wait_polls);
+    phase ^= 1u << st;
+    const uint32_t kb = base + st * 2 * block, r = rest + st * kItemBytes, im = images + (i & 1) * SPAN * 4;
+    Item cur{0, 0, 0, 0};
+    int nl = 0;
+    uint64_t lo_u = 0;
+    bool staged = false;
+    if (!producer && ok) {
+      cur = lds_item(r + kQueryBytes + kPlaceBytes);
+      nl = cur.nl();
+      staged = nl >= 1 && nl <= ml;
+      lo_u = key_lo_u + ((uint64_t)cur.b << shift);
+      if (staged) {
+        for (int m = tid; m < SPAN; m += kJoinThreads) {
+          uint32_t v = ~0u;
+          if (m < nl) {
+            const uint64_t k = biased(lds64(kb + m * 128 + ((m & 7) << 4)));
+            const uint64_t d = k <= lo_u ? 0 : (k - lo_u) >> ishift;
+            v = d > kImageMax ? kImageMax + 1 : (uint32_t)d;  // a leaf past the bucket
+          }
+          asm volatile("st.shared.u32 [%0], %1;" ::"r"(im + m * 4), "r"(v) : "memory");
+        }
+      }
+    }
     if (__syncthreads_or(!ok)) {  // a load that never landed: report, drain, stop
-      if (threadIdx.x == 0) {
+      if (tid == 0) {
         atomicOr(err, kErrTimeout);
-        for (int x = 0; x < kStages; x++)
-          if ((pending >> x) & 1u) mbar_wait_bounded(&bars[x], (phase >> x) & 1u);
-        if (!ok) mbar_wait_bounded(&bars[cur_stage], ((phase >> cur_stage) & 1u) ^ 1u);
+        for (int x = 0; x < STAGES; x++)  // every stage has loads under way but the one before st
+          if (x != (st == 0 ? STAGES - 1 : st - 1))
+            mbar_wait_bounded(&bars[x], x == st ? ((phase >> x) & 1u) ^ 1u : (phase >> x) & 1u);
       }
       __syncthreads();
       return;
     }
-    const Item cur = d[0];
-    const unsigned char *kb = base + (size_t)cur_stage * 2 * block;
-    int64_t *fs = firsts + (size_t)cur_stage * rb;
-    const bool staged = cur.nl() >= 1 && cur.nl() <= ml;
-    if (staged)
-      for (int m = threadIdx.x; m < cur.nl(); m += kThreads)
-        fs[m] = *reinterpret_cast<const int64_t *>(kb + StageTma::off(m, 0));
-    __syncthreads();
-    const StageTma st(kb, kb + block, fs);
-    int span = 1;
-    while (span < cur.nl()) span <<= 1;
-    const uint64_t lo_u = key_lo_u + ((uint64_t)cur.b << shift);
-    if (DIR && staged) {  // uniform across the CTA
-      build_dir(st, cur.nl(), span, lo_u, dshift, dir);
-      __syncthreads();
+    if (producer) {  // every thread has left the stage before
+      fill(st == 0 ? STAGES - 1 : st - 1);
+      continue;
     }
-    answer_item<LC, DIR, PLACED>(t, f, st, cur, d[1], staged, span, lo_u, dshift, dir, qs, place, out, q, qo);
-    __syncthreads();  // this stage is refilled in the next iteration
+    const int len = cur.len();
+    for (int x0 = tid; x0 < len; x0 += kJoinStep) {
+      int64_t q[kJoinQueries], v[kJoinQueries];
+      int32_t qo[kJoinQueries];
+      const bool head = x0 < kJoinStep;  // a fuller bucket's further queries are loaded here
 #pragma unroll
-    for (int x = 0; x < kStages - 1; x++) d[x] = d[x + 1];
-    d[kStages - 1] = dn;
-    cur_stage = cur_stage == kStages - 1 ? 0 : cur_stage + 1;
+      for (int j = 0; j < kJoinQueries; j++) {
+        const int y = x0 + j * kJoinThreads;
+        q[j] = kMaxKey;
+        qo[j] = -1;
+        if (y < len) {
+          qo[j] = cur.qa + y;
+          q[j] = head ? lds64(r + ((cur.qa & 1) + y) * 8) : __ldg(qs + qo[j]);
+          if constexpr (PLACED)
+            qo[j] = head ? (int32_t)lds32(r + kQueryBytes + ((cur.qa & 3) + y) * 4) : __ldg(place + qo[j]);
+        }
+      }
+      if (staged) {
+        uint32_t qi[kJoinQueries], m4[kJoinQueries];  // 4 * leaf: the last of [1, nl) whose image is <= the key's, else 0
+#pragma unroll
+        for (int j = 0; j < kJoinQueries; j++) {
+          const uint64_t qu = biased(q[j]);
+          const uint64_t d = qu <= lo_u ? 0 : (qu - lo_u) >> ishift;
+          qi[j] = d > kImageMax ? kImageMax : (uint32_t)d;
+          m4[j] = 0;
+        }
+#pragma unroll
+        for (uint32_t step = 2 * SPAN; step >= 4; step >>= 1) {
+#pragma unroll
+          for (int j = 0; j < kJoinQueries; j++)
+            if (lds32(im + m4[j] + step) <= qi[j]) m4[j] += step;
+        }
+        uint32_t row[kJoinQueries], x[kJoinQueries], c[kJoinQueries];  // c: 8 * slot
+        int64_t key[kJoinQueries];
+#pragma unroll
+        for (int j = 0; j < kJoinQueries; j++) {
+          row[j] = kb + (m4[j] << 5);
+          x[j] = (m4[j] << 2) & 0x70u;
+          c[j] = 0;
+        }
+        // the last key <= q of the leaf (Max_Key pads the tail), else slot 0
+#pragma unroll
+        for (uint32_t step = LC * 4; step >= 8; step >>= 1) {
+#pragma unroll
+          for (int j = 0; j < kJoinQueries; j++)
+            if (lds64(row[j] + ((c[j] + step) ^ x[j])) <= q[j]) c[j] += step;
+        }
+#pragma unroll
+        for (int j = 0; j < kJoinQueries; j++) key[j] = lds64(row[j] + (c[j] ^ x[j]));
+#pragma unroll
+        for (int j = 0; j < kJoinQueries; j++) {
+          while (key[j] > q[j] && row[j] != kb) {  // the image of this leaf's first key is the key's, but it lies above
+            row[j] -= 128;
+            x[j] = (x[j] - 16) & 0x70u;
+            c[j] = 0;
+            for (uint32_t step = LC * 4; step >= 8; step >>= 1)
+              if (lds64(row[j] + ((c[j] + step) ^ x[j])) <= q[j]) c[j] += step;
+            key[j] = lds64(row[j] + (c[j] ^ x[j]));
+          }
+          v[j] = HM_NOT_FOUND;
+          if (key[j] == q[j] && q[j] != kMaxKey) v[j] = lds64(row[j] + block + (c[j] ^ x[j]));
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kJoinQueries; j++) v[j] = q[j] != kMaxKey ? lookup_scalar<LC>(t, f, q[j]) : HM_NOT_FOUND;
+      }
+#pragma unroll
+      for (int j = 0; j < kJoinQueries; j++)
+        if (qo[j] >= 0) out[qo[j]] = v[j];
+    }
   }
-  // loads issued for items past the end (none are staged, but their phases
-  // must complete before the CTA's shared memory is released)
-  if (threadIdx.x == 0)
-    for (int x = 0; x < kStages; x++)
-      if ((pending >> x) & 1u) mbar_wait_bounded(&bars[x], (phase >> x) & 1u);
+  // the stages filled past the last item hold arrivals only
 }
 
-int64_t max_items(int64_t n, int nb) { return n / kItemMax + nb + 1; }
+int64_t max_items(int64_t n, int nb, int item_max) { return n / item_max + nb + 1; }
 
 int leaf_bytes(int lc) { return lc == 16 ? stage_leaf_bytes<16>() : stage_leaf_bytes<64>(); }
 
@@ -554,9 +672,7 @@ bool join_fits(const hm_tree *t) {
 
 size_t join_scratch_bytes(int64_t n, int bits) {
   const int64_t nb = (int64_t)1 << bits;
-  return (size_t)(2 * align_up(4 * (nb + 1), 256) + align_up(8 * (nb + 2), 256) +
-                  align_up((int64_t)scan_scratch_bytes(nb + 1), 256) +
-                  align_up((int64_t)sizeof(Item) * max_items(n, (int)nb), 256)) +
+  return (size_t)(align_up(4 * (nb + 1), 256) + 256 + align_up((int64_t)sizeof(Item) * max_items(n, (int)nb, std::min(kItemMin, kJoinStep)), 256)) +
          256;
 }
 
@@ -571,11 +687,8 @@ int bucket_shift(const hm_tree *t, int bits) {
 }
 
 // The leaf of each bucket boundary (nb + 1 entries): kept per tree shape in
-// the tree, else computed into leafb_scratch.  With bstart (contiguous
-// buckets) the same launch writes each bucket's item count into cnt; without
-// it the launch is skipped when the kept boundaries are valid.
-const int32_t *bucket_bounds(const hm_tree *t, int bits, int shift, const int64_t *bstart, int32_t *leafb_scratch,
-                             int32_t *cnt, cudaStream_t s) {
+// the tree, else computed into leafb_scratch.
+const int32_t *bucket_bounds(const hm_tree *t, int bits, int shift, int32_t *leafb_scratch, cudaStream_t s) {
   const int nb = 1 << bits;
   const unsigned gb = (unsigned)((nb + 1 + 255) / 256);
   int32_t *leafb = leafb_scratch;
@@ -621,9 +734,8 @@ const int32_t *bucket_bounds(const hm_tree *t, int bits, int shift, const int64_
       }
     }
   }
-  if (want_leafb || bstart) {
-    launch_pdl(bucket_prep_kernel, gb, 256, 0, s, t->view(), t->cfg.fanout, t->key_min, shift, nb, bstart, leafb,
-               bstart ? cnt : nullptr, want_leafb);
+  if (want_leafb) {
+    launch_pdl(bucket_bounds_kernel, gb, 256, 0, s, t->view(), t->cfg.fanout, t->key_min, shift, nb, leafb);
     note_launch();
   }
   if (fill_cache && cudaEventRecord(t->join_leafb_ready, s) == cudaSuccess) {
@@ -655,14 +767,15 @@ JoinKernel pick_join(int lc, bool dir) {
 using TmaJoinKernel = void (*)(const CUtensorMap, DevTree, int, const Item *, const int64_t *, const int64_t *,
                                const int32_t *, int64_t *, int, uint64_t, int, unsigned *);
 
-// The TMA join serves the binary-search variant only: with the directory
-// (thousands of queries per item) the per-lookup cost of the swizzled
-// addressing outweighs the staging work it saves (measured on 217 M queries:
-// join 1.80 against 1.58 ms; at 2^24 queries without the directory 0.336
-// against 0.347 ms).
+// The TMA join does without a directory; batches that would use one (thousands
+// of queries per bucket) take it only where measured (use_dir).
 template <bool PLACED>
-TmaJoinKernel pick_tma_join(bool dir) {
-  return dir ? nullptr : join_tma_kernel<false, PLACED>;
+TmaJoinKernel pick_tma_join(int ml) {
+  if (ml <= 32) return join_tma_kernel<PLACED, 5>;
+  if (ml <= 64) return join_tma_kernel<PLACED, 6>;
+  if (ml <= 128) return join_tma_kernel<PLACED, 7>;
+  if (ml <= 256) return join_tma_kernel<PLACED, 8>;
+  return join_tma_kernel<PLACED, 9>;
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -701,32 +814,36 @@ bool leaf_tensor_map(const hm_tree *t, CUtensorMap *m) {
 }
 
 // Shared memory of the TMA join: alignment slack, per stage a key block and a
-// value block of rb 128-B rows and rb first keys.
+// value block of rb 128-B rows, the queries, places and descriptor, and the
+// images of the first keys.
 size_t tma_join_smem(int ml) {
   const size_t rb = (size_t)((ml + 7) & ~7);
-  return 1024 + (size_t)kStages * (2 * rb * 128 + rb * 8);
+  int steps = 5;
+  while ((1 << steps) < ml) steps++;
+  return 1024 + (size_t)tma_stages(steps) * (2 * rb * 128 + kItemBytes) + (2 << steps) * 4;
 }
 
-// Launches the join over the items (their count at nitems).
-int run_join(const hm_tree *t, JoinKernel k, TmaJoinKernel tk, int bits, int64_t n_items_max, const Item *items,
-             const int64_t *nitems, const int64_t *qs, const int32_t *place, int64_t *out, int shift,
-             cudaStream_t s) {
+constexpr size_t kTmaSmem = 226 * 1024;  // of a CTA, at most
+
+// Launch the join over the items (their count at nitems).
+int run_tma_join(const hm_tree *t, TmaJoinKernel k, const CUtensorMap &tmap, int ml, int64_t n_items_max,
+                 const Item *items, const int64_t *nitems, const int64_t *qs, const int32_t *place, int64_t *out,
+                 int shift, cudaStream_t s) {
+  const size_t smem = tma_join_smem(ml);
+  const int per_sm = std::max(1, std::min(kJoinCtas, (int)((227 * 1024) / (smem + 1024))));
+  const unsigned grid = (unsigned)std::min<int64_t>(n_items_max, (int64_t)t->num_sms * per_sm);
+  int rc = opt_in_smem((const void *)k, (int)kTmaSmem);
+  if (rc) return rc;
+  launch_pdl(k, grid, kJoinThreads + 32, smem, s, tmap, t->view(), t->cfg.fanout, items, nitems, qs, place, out, ml,
+             biased(t->key_min), shift, t->d_err);
+  note_launch();
+  return HM_OK;
+}
+
+int run_join(const hm_tree *t, JoinKernel k, int ml, int64_t n_items_max, const Item *items, const int64_t *nitems,
+             const int64_t *qs, const int32_t *place, int64_t *out, int shift, cudaStream_t s) {
   if (!k) return HM_EINVAL;
-  const int lc = t->cfg.leaf_cap;
-  const int ml = stage_leaves_for(t, bits);
-  CUtensorMap tmap;
-  if (HM_JOIN_TMA && tk && leaf_tensor_map(t, &tmap)) {
-    const size_t smem = tma_join_smem(ml);
-    const int per_sm = std::max(1, std::min(8, (int)((227 * 1024) / (smem + 1024))));
-    const unsigned grid = (unsigned)std::min<int64_t>(n_items_max, (int64_t)t->num_sms * per_sm);
-    int rc = opt_in_smem((const void *)tk, (int)tma_join_smem(kStageMax / leaf_bytes(16)));
-    if (rc) return rc;
-    launch_pdl(tk, grid, kThreads, smem, s, tmap, t->view(), t->cfg.fanout, items, nitems, qs, place, out, ml,
-               biased(t->key_min), shift, t->d_err);
-    note_launch();
-    return HM_OK;
-  }
-  const size_t smem = (size_t)kStages * ml * leaf_bytes(lc);
+  const size_t smem = (size_t)kStages * ml * leaf_bytes(t->cfg.leaf_cap);
   const int per_sm = std::max(1, std::min(8, (int)((227 * 1024) / (smem + 1024))));
   const unsigned grid = (unsigned)std::min<int64_t>(n_items_max, (int64_t)t->num_sms * per_sm);
   int rc = opt_in_smem((const void *)k, kStages * kStageMax);
@@ -742,30 +859,34 @@ bool use_dir(int64_t n, int nb) { return HM_JOIN_DIR_BITS > 0 && n >= (int64_t)H
 
 }  // namespace
 
-int launch_join(const hm_tree *t, const int64_t *qs, const int64_t *bstart, int bits, int64_t n, int64_t *out,
+int launch_join(const hm_tree *t, const int64_t *qs, const uint32_t *bstart, int bits, int64_t n, int64_t *out,
                 void *scratch, cudaStream_t s, const int32_t *place) {
   if (n <= 0) return HM_OK;
   const int nb = 1 << bits;
   char *p = static_cast<char *>(scratch);
   int32_t *leafb_s = reinterpret_cast<int32_t *>(p);
   p += align_up(4 * (nb + 1), 256);
-  int32_t *cnt = reinterpret_cast<int32_t *>(p);
-  p += align_up(4 * (nb + 1), 256);
-  int64_t *first = reinterpret_cast<int64_t *>(p);
-  p += align_up(8 * (nb + 2), 256);
-  void *scan = p;
-  p += align_up((int64_t)scan_scratch_bytes(nb + 1), 256);  // keeps the 16-B items aligned
+  int64_t *n_items = reinterpret_cast<int64_t *>(p);
+  p += 256;
   Item *items = reinterpret_cast<Item *>(p);
   const int shift = bucket_shift(t, bits);
-  const unsigned gb = (unsigned)((nb + 1 + 255) / 256);
-  const int32_t *leafb = bucket_bounds(t, bits, shift, bstart, leafb_s, cnt, s);
-  exclusive_scan_i32(cnt, first, nb + 1, scan, s);
-  launch_pdl(expand_items_kernel, gb, 256, 0, s, nb, bstart, leafb, cnt, first, items);
-  note_launch();
+  const int32_t *leafb = bucket_bounds(t, bits, shift, leafb_s, s);
   const bool dir = use_dir(n, nb);
   const JoinKernel k = place ? pick_join<true>(t->cfg.leaf_cap, dir) : pick_join<false>(t->cfg.leaf_cap, dir);
-  const TmaJoinKernel tk = place ? pick_tma_join<true>(dir) : pick_tma_join<false>(dir);
-  int rc = run_join(t, k, tk, bits, max_items(n, nb), items, first + nb, qs, place, out, shift, s);
+  const int ml = stage_leaves_for(t, bits);
+  CUtensorMap tmap;
+  const bool tma = HM_JOIN_TMA && !dir && tma_join_smem(ml) <= kTmaSmem && leaf_tensor_map(t, &tmap);
+  // the TMA join takes a step of queries per item: a fuller bucket's next step
+  // is prefetched like any other item's
+  const int64_t share = n / ((int64_t)t->num_sms * 16);
+  const int item_max = tma ? kJoinStep : (int)std::min<int64_t>(kItemMax, std::max<int64_t>(kItemMin, share / kRun * kRun));
+  launch_pdl(items_kernel, (unsigned)((nb + kItemThreads - 1) / kItemThreads), kItemThreads, 0, s, nb,
+             (uint32_t)item_max, bstart, leafb, items, n_items);
+  note_launch();
+  const int64_t most = max_items(n, nb, item_max);
+  int rc = tma ? run_tma_join(t, place ? pick_tma_join<true>(ml) : pick_tma_join<false>(ml), tmap, ml, most, items,
+                              n_items, qs, place, out, shift, s)
+               : run_join(t, k, ml, most, items, n_items, qs, place, out, shift, s);
   if (rc) return rc;
   return cuda_err(cudaGetLastError());
 }

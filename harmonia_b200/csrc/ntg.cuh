@@ -111,8 +111,8 @@ __device__ __forceinline__ bool stage_top(const DevTree &t, unsigned char *smem,
     mbar_init(bar, 1);
     fence_mbar_init();
     mbar_expect_tx(bar, rows_bytes + pref_bytes);
-    bulk_g2s(smem, t.inner, rows_bytes, bar);
-    bulk_g2s(smem + rows_bytes, t.prefix, pref_bytes, bar);
+    bulk_g2s(smem_addr(smem), t.inner, rows_bytes, bar);
+    bulk_g2s(smem_addr(smem + rows_bytes), t.prefix, pref_bytes, bar);
   }
   __syncthreads();
   if (mbar_wait_bounded(bar, 0, t.wait_polls)) return true;
