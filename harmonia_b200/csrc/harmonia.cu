@@ -539,7 +539,7 @@ int run_planned_search(hm_tree *t, const SearchPlan &p, const int64_t *d_q, int6
     rc = launch_join(t, qs, bstart, p.bits, n, res, js, s);
     prof_end(t, kStageJoin, tok, s);
   } else {
-    SearchLaunch l{qs, res, nullptr, n};
+    SearchLaunch l{qs, res, nullptr, n, true};
     rc = launch_search(t, l, t->cfg.group_width, t->cfg.queries_per_group, s);
     prof_end(t, kStageSearch, tok, s);
   }

@@ -97,6 +97,6 @@ extern "C" int hm_search_noalloc(hm_tree *t, const int64_t *q, size_t n_, int64_
   cudaStream_t s = reinterpret_cast<cudaStream_t>(hs);
   rc = partition_queries(t, q, n, kBits, qs, pos, ps, s);
   if (rc) return rc;
-  SearchLaunch l{qs, out, pos, n};
+  SearchLaunch l{qs, out, pos, n, true};
   return launch_search(t, l, t->cfg.group_width, t->cfg.queries_per_group, s);
 }

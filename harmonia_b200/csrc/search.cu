@@ -224,6 +224,7 @@ __device__ __forceinline__ void search_tile(const DevTree &t, const int64_t *sro
 
 template <int W, int F, int LC, int Q>
 __global__ void __launch_bounds__(kThreads, (Q <= 2 ? HM_SEARCH_MINB : 1)) search_kernel(Args a) {
+  pdl_enter();
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int TILE = (kThreads / W) * Q;
   const DevTree &t = a.t;
@@ -373,7 +374,10 @@ int launch_search(const hm_tree *t, const SearchLaunch &l, int group_width, int 
   a.n = l.n;
   a.nb = 0;
   a.err = t->d_err;
-  fn<<<blocks, kThreads, smem, s>>>(a);
+  if (l.after_partition)
+    fn<<<blocks, kThreads, smem, s>>>(a);
+  else
+    launch_pdl(fn, blocks, kThreads, smem, s, a);
   note_launch();
   return cuda_err(cudaGetLastError());
 }
