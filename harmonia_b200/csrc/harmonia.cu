@@ -152,6 +152,70 @@ void release_after(void *p, cudaStream_t s) {
   dev_release(p);
 }
 
+// ---- small results to the host ----
+// Page-locked slots that the device maps, handed out to one call at a time.
+// They are made kSlotChunk at a time when all are in use (a few calls run at
+// once; 256 B each) and kept for the process; hm_trim_memory frees them when
+// none is in use.
+namespace {
+constexpr size_t kSlot = 256;
+constexpr int kSlotChunk = 64;
+std::mutex g_slot_mu;
+std::vector<char *> g_slots;        // free ones
+std::vector<void *> g_slot_chunks;  // the allocations
+
+char *take_slot() {
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  if (g_slots.empty()) {
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, kSlot * kSlotChunk, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    g_slot_chunks.push_back(p);
+    for (int i = 0; i < kSlotChunk; i++) g_slots.push_back(static_cast<char *>(p) + i * kSlot);
+  }
+  char *c = g_slots.back();
+  g_slots.pop_back();
+  return c;
+}
+
+void give_slot(char *p) {
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  g_slots.push_back(p);
+}
+
+void trim_slots() {
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  if (g_slots.size() != g_slot_chunks.size() * kSlotChunk) return;
+  for (void *p : g_slot_chunks) cudaFreeHost(p);
+  g_slot_chunks.clear();
+  g_slots.clear();
+}
+
+__global__ void publish_kernel(uint32_t *host, const uint32_t *src, int words, const unsigned *d_err, int err_at) {
+  pdl_enter();
+  for (int i = threadIdx.x; i < words; i += 32) host[i] = src[i];
+  if (d_err && threadIdx.x == 0) host[err_at] = *d_err;
+}
+}  // namespace
+
+int read_back(void *dst, const void *src, size_t bytes, cudaStream_t s, const unsigned *d_err, unsigned *err) {
+  char *slot = take_slot();
+  if (!slot) return HM_ENOMEM;
+  const int err_at = (int)(kReadBack / 4);
+  cudaError_t e = launch_pdl(publish_kernel, 1, 32, 0, s, reinterpret_cast<uint32_t *>(slot),
+                             static_cast<const uint32_t *>(src), (int)(bytes / 4), d_err, err_at);
+  note_launch();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) {
+    std::memcpy(dst, slot, bytes);
+    if (err) std::memcpy(err, slot + kReadBack, 4);
+  }
+  give_slot(slot);
+  return cuda_err(e);
+}
+
 // Scratch blocks come from the block cache above and grow by half again when
 // a call needs more.  An outgrown block is retired, not released: its last
 // use may still run on another stream, and waiting for it would stall that
@@ -446,6 +510,13 @@ int ensure_pinned(hm_tree *t, size_t bytes) {
   return HM_OK;
 }
 
+// The code of a recorded error word, which is cleared.
+int take_error(hm_tree *t, unsigned err, hm_stream hs) {
+  cudaMemsetAsync(t->d_err, 0, 4, as_stream(hs));
+  cudaStreamSynchronize(as_stream(hs));
+  return (err & kErrTimeout) ? HM_ETIMEOUT : HM_ECUDA;
+}
+
 // Search of device-resident queries on stream s by the plan for n queries.
 int search_device(hm_tree *t, const int64_t *d_q, int64_t n, int64_t *d_out, cudaStream_t s,
                   void *scratch_base, size_t scratch_avail) {
@@ -709,9 +780,8 @@ int hm_bulk_load(const int64_t *keys, const int64_t *vals, size_t n_, const hm_c
     rc = build_from_pairs(t->target(), in_k, in_v, n, reinterpret_cast<int64_t *>(uk_alt), vv_alt,
                           reinterpret_cast<int64_t *>(uk), vv, sort_scratch, t->num_sms, &ctl, s);
     if (rc == HM_OK) {
-      e = cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-      rc = cuda_err(e);
+      static_assert(sizeof(h) <= kReadBack, "one read");
+      rc = read_back(&h, ctl, sizeof(h), s);
     }
     if (rc == HM_OK && !h.skew && h.flags) rc = (h.flags & 2u) ? HM_EMAXKEY : HM_EDUPLICATE;
     if (rc || !h.skew) {
@@ -940,26 +1010,28 @@ int hm_search(hm_tree *t, const int64_t *q, size_t n_, int64_t *out, hm_stream h
 
 int hm_trim_memory(size_t *released) {
   const size_t freed = trim_cache(-1);
+  trim_slots();
   if (released) *released = freed;
   return HM_OK;
 }
 
 int hm_sync(hm_tree *t, hm_stream hs) {
   if (!t) return HM_EINVAL;
-  cudaError_t e = cudaStreamSynchronize(as_stream(hs));
-  if (e != cudaSuccess) return cuda_err(e);
   // the error word is read on the caller's stream (the legacy default stream
   // would also wait for other streams' work on this device)
   unsigned err = 0;
-  e = cudaMemcpyAsync(&err, t->d_err, 4, cudaMemcpyDeviceToHost, as_stream(hs));
-  if (e == cudaSuccess) e = cudaStreamSynchronize(as_stream(hs));
-  if (e != cudaSuccess) return cuda_err(e);
-  if (err) {
-    cudaMemsetAsync(t->d_err, 0, 4, as_stream(hs));
-    cudaStreamSynchronize(as_stream(hs));
-    return (err & kErrTimeout) ? HM_ETIMEOUT : HM_ECUDA;
+  int dev = -1;
+  cudaGetDevice(&dev);
+  if (dev == t->device) {
+    int rc = read_back(&err, t->d_err, 4, as_stream(hs));
+    if (rc) return rc;
+  } else {  // no kernel of the current device can follow the stream
+    cudaError_t e = cudaStreamSynchronize(as_stream(hs));
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&err, t->d_err, 4, cudaMemcpyDeviceToHost, as_stream(hs));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(as_stream(hs));
+    if (e != cudaSuccess) return cuda_err(e);
   }
-  return HM_OK;
+  return err ? take_error(t, err, hs) : HM_OK;
 }
 
 int hm_export(hm_tree *t, int64_t *keys, int64_t *vals, size_t cap, size_t *n) {
@@ -991,98 +1063,148 @@ int hm_export(hm_tree *t, int64_t *keys, int64_t *vals, size_t cap, size_t *n) {
 
 namespace {
 
-// Body of hm_range (len given, end == nullptr) and hm_range_between (end
-// given, len == nullptr): locate, scan of the counts into offsets, total to
-// the host, compacted copy.
-int range_impl(hm_tree *t, const int64_t *start, const int32_t *len, const int64_t *end, size_t n_,
-               int64_t *offsets, int64_t *okeys, int64_t *ovals, size_t cap, size_t *total, hm_stream hs) {
-  const int64_t n = (int64_t)n_;
-  cudaStream_t s = as_stream(hs);
-  if (total) *total = 0;
+}  // namespace
+
+// The first half of a range scan: where each query's records lie and where
+// they go, until the caller has a place for them.
+struct hm_range_scan {
+  hm_tree *t;
+  hm_stream hs;
+  ScratchLease lease;
+  int64_t n;
+  int32_t *leaf = nullptr, *slot = nullptr;
+  int64_t *off = nullptr;  // device
+  int64_t total = 0;
+  int tok = -1;
+  hm_range_scan(hm_tree *tree, hm_stream s, int64_t count) : t(tree), hs(s), lease(tree, as_stream(s)), n(count) {}
+};
+
+namespace {
+
+// Locate (len given, end == nullptr: the first len records; end given: up to
+// end) and scan of the counts into the offsets, on the device; enqueues only.
+int range_enqueue(hm_range_scan *r, const int64_t *start, const int32_t *len, const int64_t *end, int64_t *offsets,
+                  bool dev_out) {
+  hm_tree *t = r->t;
+  cudaStream_t s = as_stream(r->hs);
+  const int64_t n = r->n;
   const void *second = end ? static_cast<const void *>(end) : static_cast<const void *>(len);
   const bool dev_in = n == 0 || (is_device_ptr(start) && is_device_ptr(second));
-  const bool dev_out = is_device_ptr(offsets);
   const size_t b8 = (size_t)align_up((n + 1) * 8, 256), b4 = (size_t)align_up(n * 4 + 4, 256);
-  size_t need = 2 * b4 + b8 + (size_t)align_up((int64_t)scan_scratch_bytes(n + 1), 256);
+  const size_t scan_bytes = (size_t)align_up((int64_t)scan_scratch_bytes(n + 1), 256);
+  size_t need = 2 * b4 + b8 + scan_bytes;
   if (!dev_in) need += b8 + (end ? b8 : b4);
   if (!dev_out) need += b8;
-  ScratchLease lease(t, s);
-  int rc = lease.acquire(need);
+  int rc = r->lease.acquire(need);
   if (rc) return rc;
-  char *p = static_cast<char *>(lease.ptr());
-  int32_t *fl = reinterpret_cast<int32_t *>(p);
-  p += b4;
-  int32_t *fs = reinterpret_cast<int32_t *>(p);
-  p += b4;
-  int64_t *cnt = reinterpret_cast<int64_t *>(p);
-  p += b8;
-  void *scan_scratch = p;
-  p += align_up((int64_t)scan_scratch_bytes(n + 1), 256);
-  const int64_t *d_start = start;
-  const int32_t *d_len = len;
-  const int64_t *d_end = end;
-  cudaError_t e = cudaSuccess;
+  char *p = static_cast<char *>(r->lease.ptr());
+  auto take = [&](size_t b) { char *x = p; p += b; return x; };
+  r->leaf = reinterpret_cast<int32_t *>(take(b4));
+  r->slot = reinterpret_cast<int32_t *>(take(b4));
+  int64_t *cnt = reinterpret_cast<int64_t *>(take(b8));
+  void *scan_scratch = take(scan_bytes);
   if (!dev_in) {
-    int64_t *ds = reinterpret_cast<int64_t *>(p);
-    p += b8;
-    e = cudaMemcpyAsync(ds, start, n * 8, cudaMemcpyHostToDevice, s);
-    d_start = ds;
+    int64_t *ds = reinterpret_cast<int64_t *>(take(b8));
+    cudaError_t e = cudaMemcpyAsync(ds, start, n * 8, cudaMemcpyHostToDevice, s);
+    start = ds;
     if (end) {
-      int64_t *de = reinterpret_cast<int64_t *>(p);
-      p += b8;
+      int64_t *de = reinterpret_cast<int64_t *>(take(b8));
       if (e == cudaSuccess) e = cudaMemcpyAsync(de, end, n * 8, cudaMemcpyHostToDevice, s);
-      d_end = de;
+      end = de;
     } else {
-      int32_t *dl = reinterpret_cast<int32_t *>(p);
-      p += b4;
+      int32_t *dl = reinterpret_cast<int32_t *>(take(b4));
       if (e == cudaSuccess) e = cudaMemcpyAsync(dl, len, n * 4, cudaMemcpyHostToDevice, s);
-      d_len = dl;
+      len = dl;
     }
     if (e != cudaSuccess) return cuda_err(e);
   }
-  int64_t *d_off = dev_out ? offsets : reinterpret_cast<int64_t *>(p);
-  const int tok = prof_begin(t, s);
+  r->off = dev_out ? offsets : reinterpret_cast<int64_t *>(p);
+  r->tok = prof_begin(t, s);
   if (n > 0) {
-    rc = range_locate(t, d_start, d_len, d_end, n, fl, fs, cnt, s);
+    rc = range_locate(t, start, len, end, n, r->leaf, r->slot, cnt, s);
     if (rc) return rc;
   }
-  exclusive_scan_i64(cnt, d_off, n, scan_scratch, s);
-  int64_t tot = 0;
-  e = cudaMemcpyAsync(&tot, d_off + n, 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_err(e);
-  if (total) *total = (size_t)tot;
-  if (!dev_out) {
-    e = cudaMemcpyAsync(offsets, d_off, (n + 1) * 8, cudaMemcpyDeviceToHost, s);
+  exclusive_scan_i64(cnt, r->off, n, scan_scratch, s);
+  return cuda_err(cudaGetLastError());
+}
+
+// Waits for the locate and the scan: the total, the offsets in host memory if
+// the caller's are there, and any error the locate's staging recorded.
+int range_total(hm_range_scan *r, int64_t *host_offsets) {
+  hm_tree *t = r->t;
+  cudaStream_t s = as_stream(r->hs);
+  unsigned err = 0;
+  int rc = read_back(&r->total, r->off + r->n, 8, s, t->d_err, &err);
+  if (rc) return rc;
+  if (host_offsets) {
+    cudaError_t e = cudaMemcpyAsync(host_offsets, r->off, (r->n + 1) * 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_err(e);
   }
-  if ((size_t)tot > cap) return HM_ECAPACITY;
-  if (tot == 0) return HM_OK;
-  if (!okeys || !ovals) return HM_EINVAL;
-  const bool dev_rec = is_device_ptr(okeys) && is_device_ptr(ovals);
-  if (dev_rec) {
-    rc = range_copy_out(t, fl, fs, d_off, n, (int64_t)cap, okeys, ovals, s);
-    prof_end(t, kStageRange, tok, s);
-    if (rc) return rc;
-    return hm_sync(t, hs);
+  return err ? take_error(t, err, r->hs) : HM_OK;
+}
+
+// The records into okeys and ovals, which hold them all; returns when done.
+int range_records(hm_range_scan *r, int64_t *okeys, int64_t *ovals) {
+  hm_tree *t = r->t;
+  cudaStream_t s = as_stream(r->hs);
+  const int64_t tot = r->total;
+  if (is_device_ptr(okeys) && is_device_ptr(ovals)) {
+    int rc = range_copy_out(t, r->leaf, r->slot, r->off, r->n, tot, okeys, ovals, s);
+    prof_end(t, kStageRange, r->tok, s);
+    return rc ? rc : cuda_err(cudaStreamSynchronize(s));
   }
   // host record buffers: a stream-ordered temporary (no device-wide
   // synchronisation, unlike cudaMalloc/cudaFree)
   int64_t *tk = nullptr;
-  e = cudaMallocAsync(reinterpret_cast<void **>(&tk), 2 * (size_t)align_up(tot * 8, 256), s);
+  cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&tk), 2 * (size_t)align_up(tot * 8, 256), s);
   if (e != cudaSuccess) return cuda_err(e);
   int64_t *tv = reinterpret_cast<int64_t *>(reinterpret_cast<char *>(tk) + align_up(tot * 8, 256));
-  rc = range_copy_out(t, fl, fs, d_off, n, tot, tk, tv, s);
-  prof_end(t, kStageRange, tok, s);
+  int rc = range_copy_out(t, r->leaf, r->slot, r->off, r->n, tot, tk, tv, s);
+  prof_end(t, kStageRange, r->tok, s);
   if (rc == HM_OK) {
     e = cudaMemcpyAsync(okeys, tk, tot * 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ovals, tv, tot * 8, cudaMemcpyDeviceToHost, s);
   }
   cudaFreeAsync(tk, s);
   if (rc == HM_OK && e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (rc == HM_OK) rc = cuda_err(e);
-  return rc ? rc : hm_sync(t, hs);
+  return rc ? rc : cuda_err(e);
+}
+
+// Body of hm_range (len given, end == nullptr) and hm_range_between (end
+// given, len == nullptr).
+int range_impl(hm_tree *t, const int64_t *start, const int32_t *len, const int64_t *end, size_t n,
+               int64_t *offsets, int64_t *okeys, int64_t *ovals, size_t cap, size_t *total, hm_stream hs) {
+  hm_range_scan r(t, hs, (int64_t)n);
+  const bool dev_out = is_device_ptr(offsets);
+  int rc = range_enqueue(&r, start, len, end, offsets, dev_out);
+  if (rc) return rc;
+  rc = range_total(&r, dev_out ? nullptr : offsets);
+  if (total) *total = (size_t)r.total;
+  if (rc) return rc;
+  if ((size_t)r.total > cap) return HM_ECAPACITY;
+  if (r.total == 0) return HM_OK;
+  if (!okeys || !ovals) return HM_EINVAL;
+  return range_records(&r, okeys, ovals);
+}
+
+int range_begin(hm_tree *t, const int64_t *start, const int32_t *len, const int64_t *end, size_t n, int64_t *offsets,
+                size_t *total, hm_stream hs, hm_range_scan **scan) {
+  if (total) *total = 0;
+  if (scan) *scan = nullptr;
+  if (!t || !scan || (n > 0 && (!start || (!len && !end))) || !offsets) return HM_EINVAL;
+  hm_range_scan *r = new (std::nothrow) hm_range_scan(t, hs, (int64_t)n);
+  if (!r) return HM_ENOMEM;
+  const bool dev_out = is_device_ptr(offsets);
+  int rc = range_enqueue(r, start, len, end, offsets, dev_out);
+  if (rc == HM_OK) rc = range_total(r, dev_out ? nullptr : offsets);
+  if (rc) {
+    delete r;
+    return rc;
+  }
+  if (total) *total = (size_t)r->total;
+  *scan = r;
+  return HM_OK;
 }
 
 }  // namespace
@@ -1101,6 +1223,24 @@ int hm_range_between(hm_tree *t, const int64_t *start, const int64_t *end, size_
   if (total) *total = 0;
   if (!t || (n > 0 && (!start || !end)) || !offsets) return HM_EINVAL;
   return range_impl(t, start, nullptr, end, n, offsets, okeys, ovals, cap, total, hs);
+}
+
+int hm_range_begin(hm_tree *t, const int64_t *start, const int32_t *len, size_t n, int64_t *offsets, size_t *total,
+                   hm_stream hs, hm_range_scan **scan) {
+  return range_begin(t, start, len, nullptr, n, offsets, total, hs, scan);
+}
+
+int hm_range_between_begin(hm_tree *t, const int64_t *start, const int64_t *end, size_t n, int64_t *offsets,
+                           size_t *total, hm_stream hs, hm_range_scan **scan) {
+  return range_begin(t, start, nullptr, end, n, offsets, total, hs, scan);
+}
+
+int hm_range_finish(hm_range_scan *scan, int64_t *okeys, int64_t *ovals) {
+  if (!scan) return HM_EINVAL;
+  int rc = HM_OK;
+  if (okeys && ovals && scan->total > 0) rc = range_records(scan, okeys, ovals);
+  delete scan;
+  return rc;
 }
 
 int hm_delete_batch(hm_tree *t, const int64_t *keys, size_t n_, size_t *removed, hm_stream hs) {
@@ -1127,7 +1267,7 @@ int hm_delete_batch(hm_tree *t, const int64_t *keys, size_t n_, size_t *removed,
   prof_end(t, kStageDelete, tok, s);
   if (removed) *removed = (size_t)gone;
   choose_smem_levels(t);
-  return rc || !err ? rc : hm_sync(t, hs);
+  return rc || !err ? rc : take_error(t, err, hs);
 }
 
 int hm_upsert_batch(hm_tree *t, const int64_t *keys, const int64_t *vals, size_t n_, int flags,
@@ -1156,7 +1296,7 @@ int hm_upsert_batch(hm_tree *t, const int64_t *keys, const int64_t *vals, size_t
   int rc = upsert_epoch(t, dk, dv, n, flags, &err, s);
   prof_end(t, kStageUpsert, tok, s);
   choose_smem_levels(t);
-  return rc || !err ? rc : hm_sync(t, hs);
+  return rc || !err ? rc : take_error(t, err, hs);
 }
 
 int hm_autotune(hm_tree *t, const int64_t *sample_q, size_t n_, hm_config *best) {

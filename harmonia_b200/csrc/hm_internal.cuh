@@ -474,6 +474,15 @@ cudaError_t dev_alloc(void **p, size_t bytes);
 void dev_release(void *p);
 void release_after(void *p, cudaStream_t s);
 
+// ---- small results to the host (harmonia.cu) ----
+// Waits for stream s and brings `bytes` (at most kReadBack) of device memory at
+// src to dst and, if err is given, the word at d_err to *err.  A one-warp
+// kernel writes them to page-locked memory that the device maps, so the call
+// costs one wait and no copy through the driver's staging.
+constexpr size_t kReadBack = 192;
+int read_back(void *dst, const void *src, size_t bytes, cudaStream_t s, const unsigned *d_err = nullptr,
+              unsigned *err = nullptr);
+
 // ---- misc ----
 int cuda_err(cudaError_t e);
 

@@ -406,7 +406,9 @@ int range_locate(const hm_tree *t, const int64_t *start, const int32_t *len, con
   }
   const int64_t per = end ? kThreads / 8 : kThreads / 4;
   const unsigned grid = (unsigned)std::min<int64_t>((n + per - 1) / per, (int64_t)t->num_sms * 6);
-  k<<<grid, kThreads, smem, s>>>(t->view(), start, len, end, n, first_leaf, first_slot, count, t->d_err);
+  DevTree v = t->view();
+  v.wait_polls = kSpinLimit;  // hm_set_wait_limit is for the point searches
+  k<<<grid, kThreads, smem, s>>>(v, start, len, end, n, first_leaf, first_slot, count, t->d_err);
   note_launch();
   return cuda_err(cudaGetLastError());
 }

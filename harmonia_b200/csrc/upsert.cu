@@ -869,10 +869,8 @@ struct Epoch {
   }
 
   int read(bsort::Ctl *h, cudaStream_t s) const {
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, ctl, sizeof(*h), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    return cuda_err(e);
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? cuda_err(e) : read_back(h, ctl, sizeof(*h), s);
   }
 };
 

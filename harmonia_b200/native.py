@@ -30,7 +30,8 @@ EXPORTS = (
     "hm_search_noalloc", "hm_server_config_default", "hm_server_start", "hm_server_submit",
     "hm_server_wait", "hm_server_get_stats", "hm_server_reset_stats", "hm_server_stop", "hm_server_free",
     "hm_last_cuda_error", "hm_read_keys", "hm_read_ranges", "hm_write_keys", "hm_snapshot_save",
-    "hm_snapshot_load", "hm_delete_batch", "hm_search_baseline", "hm_trim_memory",
+    "hm_snapshot_load", "hm_delete_batch", "hm_search_baseline", "hm_trim_memory", "hm_range_begin", "hm_range_between_begin",
+    "hm_range_finish",
 )
 HM_NOALLOC_MAX_QUERIES = 1 << 20
 
@@ -98,6 +99,9 @@ def lib() -> ctypes.CDLL:
     L.hm_search_batches.argtypes = [P, ctypes.POINTER(Batch), I, P]
     L.hm_range.argtypes = [P, P, P, SZ, P, P, P, SZ, ctypes.POINTER(SZ), P]
     L.hm_range_between.argtypes = [P, P, P, SZ, P, P, P, SZ, ctypes.POINTER(SZ), P]
+    L.hm_range_begin.argtypes = [P, P, P, SZ, P, ctypes.POINTER(SZ), P, PT]
+    L.hm_range_between_begin.argtypes = [P, P, P, SZ, P, ctypes.POINTER(SZ), P, PT]
+    L.hm_range_finish.argtypes = [P, P, P]
     L.hm_upsert_batch.argtypes = [P, P, P, SZ, I, P]
     L.hm_export.argtypes = [P, P, P, SZ, ctypes.POINTER(SZ)]
     L.hm_tree_get_info.argtypes = [P, ctypes.POINTER(TreeInfo)]

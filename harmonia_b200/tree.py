@@ -24,6 +24,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 
 import numpy as np
 
@@ -82,6 +83,7 @@ class BPlusTree:
 
     def __init__(self, handle: int):
         self._h = ctypes.c_void_p(handle)
+        self._search = lib().hm_search
 
     # ---- construction ----
     @classmethod
@@ -151,6 +153,18 @@ class BPlusTree:
 
     # ---- queries ----
     def search(self, keys, out=None, stream=None):
+        torch = sys.modules.get("torch")
+        if torch is not None and type(keys) is torch.Tensor and keys.dtype is torch.int64 and keys.dim() == 1 \
+                and keys.is_contiguous():
+            # the usual call, with little in front of the launch: it is most of a small batch's time
+            if out is None:
+                out = torch.empty_like(keys)
+            n = keys.shape[0]
+            if n:
+                rc = self._search(self._h, keys.data_ptr(), n, _ptr(out), None if stream is None else _stream_ptr(stream))
+                if rc:
+                    check(rc, "hm_search")
+            return out
         keys = _as_i64(keys)
         n = len(keys)
         if out is None:
@@ -187,46 +201,37 @@ class BPlusTree:
         """Returns (offsets[n+1], keys, values): query i owns [offsets[i], offsets[i+1])."""
         start = _as_i64(start)
         length = _as_i32(length)
-        n = len(start)
-        offsets = _empty_like(start, n + 1)
-        cap = int(length.clip(min=0).sum()) if n else 0
-        okeys = _empty_like(start, max(cap, 1))
-        ovals = _empty_like(start, max(cap, 1))
-        total = ctypes.c_size_t()
-        check(lib().hm_range(self._h, _ptr(start) if n else None, _ptr(length) if n else None, n,
-                             _ptr(offsets), _ptr(okeys), _ptr(ovals), cap, ctypes.byref(total),
-                             _stream_ptr(stream)), "hm_range")
-        m = total.value
-        return offsets, okeys[:m], ovals[:m]
+        return self._range(lib().hm_range_begin, "hm_range", start, length, stream)
 
     def range_between(self, start, end, cap=None, stream=None):
         """Inclusive ranges, as the reference's BPlusTree::range_search:
         every record with start[i] <= key <= end[i].  Returns (offsets[n+1],
-        keys, values).  cap bounds the record count (default: counted by a
-        first call that returns HM_ECAPACITY with the total)."""
+        keys, values).  cap bounds the record count (default: as many as there
+        are)."""
         start = _as_i64(start)
         end = _as_i64(end)
         if len(start) != len(end):
             raise ValueError("start and end differ in length")
+        return self._range(lib().hm_range_between_begin, "hm_range_between", start, end, stream, cap)
+
+    def _range(self, begin, what, start, second, stream, cap=None):
         n = len(start)
         offsets = _empty_like(start, n + 1)
         total = ctypes.c_size_t()
-
-        def call(c, ok, ov):
-            return lib().hm_range_between(self._h, _ptr(start) if n else None, _ptr(end) if n else None, n,
-                                          _ptr(offsets), _ptr(ok) if ok is not None else None,
-                                          _ptr(ov) if ov is not None else None, c, ctypes.byref(total),
-                                          _stream_ptr(stream))
-
-        if cap is None:
-            rc = call(0, None, None)
-            if rc not in (0, native.HM_ECAPACITY):
-                check(rc, "hm_range_between")
-            cap = total.value
-        okeys = _empty_like(start, max(cap, 1))
-        ovals = _empty_like(start, max(cap, 1))
-        check(call(cap, okeys, ovals), "hm_range_between")
+        scan = ctypes.c_void_p()
+        check(begin(self._h, _ptr(start) if n else None, _ptr(second) if n else None, n, _ptr(offsets),
+                    ctypes.byref(total), _stream_ptr(stream), ctypes.byref(scan)), what)
         m = total.value
+        try:
+            if cap is not None and m > cap:
+                check(native.HM_ECAPACITY, what)
+            okeys = _empty_like(start, max(m, 1))
+            ovals = _empty_like(start, max(m, 1))
+            held, scan.value = scan.value, None
+            check(lib().hm_range_finish(held, _ptr(okeys), _ptr(ovals)), what)
+        finally:
+            if scan.value:  # not finished: free it
+                lib().hm_range_finish(scan.value, None, None)
         return offsets, okeys[:m], ovals[:m]
 
     # ---- updates ----

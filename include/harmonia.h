@@ -183,6 +183,20 @@ int hm_range_between(hm_tree *t, const int64_t *start, const int64_t *end, size_
                      int64_t *offsets, int64_t *okeys, int64_t *ovals, size_t cap,
                      size_t *total, hm_stream s);
 
+/* A range scan in two halves, for callers that allocate the record buffers
+ * once they know how many records there are: the begin calls do everything but
+ * the copy of the records (offsets and *total as hm_range) and return a scan,
+ * which hm_range_finish completes into buffers of at least *total records and
+ * frees (with okeys or ovals NULL it only frees).  The scan holds a scratch
+ * block of the tree; finish it before the tree changes or is freed, offsets
+ * unchanged, and order other streams' work on the buffers after the call. */
+typedef struct hm_range_scan hm_range_scan;
+int hm_range_begin(hm_tree *t, const int64_t *start, const int32_t *len, size_t n,
+                   int64_t *offsets, size_t *total, hm_stream s, hm_range_scan **scan);
+int hm_range_between_begin(hm_tree *t, const int64_t *start, const int64_t *end, size_t n,
+                           int64_t *offsets, size_t *total, hm_stream s, hm_range_scan **scan);
+int hm_range_finish(hm_range_scan *scan, int64_t *okeys, int64_t *ovals);
+
 #define HM_UPSERT_SUPPLIED 0        /* an existing key takes the supplied value */
 #define HM_UPSERT_REF_KEY_MINUS_1 1 /* an existing key takes key-1, as the reference does */
 

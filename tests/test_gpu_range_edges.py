@@ -40,3 +40,33 @@ def test_chunk_edges(n, cfg):
         for cap in (None, int(exp[0][-1])):
             got = t.range_between(cuda(start), cuda(end), cap=cap)
             assert all((a.cpu().numpy() == b).all() for a, b in zip(got, exp))
+
+
+def test_scan_in_two_halves():
+    """Scans begun and dropped give their scratch back, host and device buffers alike."""
+    import ctypes
+
+    from harmonia_b200 import HarmoniaError, native
+
+    keys = dg.gen_keys(5000, seed=3)
+    sk = np.sort(keys)
+    with BPlusTree.bulk_load(keys, dg.values_for(keys)) as t:
+        tree = po.PortTree(sk, dg.values_for(sk))
+        start = np.ascontiguousarray(sk[::50])
+        end = start + 2**55
+        exp = tree.range_between(start, end)
+        for s, e in ((start, end), (cuda(start), cuda(end))):
+            off = np.zeros(len(start) + 1, np.int64) if s is start else torch.zeros(len(start) + 1, dtype=torch.int64, device="cuda")
+            ptr = (lambda a: a.ctypes.data) if s is start else (lambda a: a.data_ptr())
+            for _ in range(20):  # more scans than the scratch pool keeps blocks
+                scan, total = ctypes.c_void_p(), ctypes.c_size_t()
+                native.check(native.lib().hm_range_between_begin(t.handle, ptr(s), ptr(e), len(start), ptr(off),
+                                                                 ctypes.byref(total), None, ctypes.byref(scan)))
+                assert total.value == exp[0][-1]
+                native.check(native.lib().hm_range_finish(scan, None, None))
+            with pytest.raises(HarmoniaError) as err:
+                t.range_between(s, e, cap=int(exp[0][-1]) - 1)
+            assert err.value.code == native.HM_ECAPACITY
+            got = t.range_between(s, e)
+            assert all((np.asarray(a.cpu() if hasattr(a, "cpu") else a) == b).all() for a, b in zip(got, exp))
+        assert native.lib().hm_range_finish(None, None, None) == -1
