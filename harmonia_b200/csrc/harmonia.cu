@@ -585,15 +585,19 @@ int run_planned_search(hm_tree *t, const SearchPlan &p, const int64_t *d_q, int6
   int64_t *res = reinterpret_cast<int64_t *>(b + align_up(n * 8, 256));
   char *ps = b + 2 * align_up(n * 8, 256);
   char *js = ps + partition_scratch_bytes(n, p.bits, true, p.batches);
-  const uint32_t *bstart = nullptr;
+  JoinItems ji;
+  if (p.join) {
+    int rc = prepare_join(t, p.bits, n, js, s, &ji);
+    if (rc) return rc;
+  }
   if (p.placed) {  // the join places results in first-pass order: one inverse pass
     int32_t *place = reinterpret_cast<int32_t *>(js + join_scratch_bytes(n, p.bits));
     int tok = prof_begin(t, s);
-    int rc = partition_queries_placed(t, d_q, n, p.bits, qs, place, ps, s, &bstart, bv);
+    int rc = partition_queries_placed(t, d_q, n, p.bits, qs, place, ps, s, &ji, bv);
     prof_end(t, kStagePartition, tok, s);
     if (rc) return rc;
     tok = prof_begin(t, s);
-    rc = launch_join(t, qs, bstart, p.bits, n, res, js, s, place);
+    rc = launch_join(t, qs, p.bits, n, res, ji, s, place);
     prof_end(t, kStageJoin, tok, s);
     if (rc) return rc;
     tok = prof_begin(t, s);
@@ -602,12 +606,12 @@ int run_planned_search(hm_tree *t, const SearchPlan &p, const int64_t *d_q, int6
     return rc;
   }
   int tok = prof_begin(t, s);
-  int rc = partition_queries(t, d_q, n, p.bits, qs, nullptr, ps, s, &bstart, bv);
+  int rc = partition_queries(t, d_q, n, p.bits, qs, nullptr, ps, s, p.join ? &ji : nullptr, bv);
   prof_end(t, kStagePartition, tok, s);
   if (rc) return rc;
   tok = prof_begin(t, s);
   if (p.join) {
-    rc = launch_join(t, qs, bstart, p.bits, n, res, js, s);
+    rc = launch_join(t, qs, p.bits, n, res, ji, s);
     prof_end(t, kStageJoin, tok, s);
   } else {
     SearchLaunch l{qs, res, nullptr, n, true};

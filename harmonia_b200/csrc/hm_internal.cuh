@@ -334,6 +334,27 @@ int search_tile_queries(int group_width, int qpg);  // queries per CTA tile
 int launch_search_warm(const hm_tree *t, int group_width, int qpg);
 size_t search_smem_bytes(const hm_tree *t);
 
+// ---- work items of the bucket join ----
+// A work item: some queries of one bucket, grouped queries
+// [qa, qa + len), and the bucket's leaves [l0, l0 + nl); the leaves are
+// staged once for all of them.
+struct __align__(16) Item {
+  int32_t qa, l0, b;  // first query, first leaf, bucket
+  uint32_t len_nl;    // queries << 16 | leaves (capped at 65535)
+  __host__ __device__ int len() const { return (int)(len_nl >> 16); }
+  __host__ __device__ int nl() const { return (int)(len_nl & 0xffffu); }
+};
+
+// Where the pre-sort's scan of its buckets writes the join's work items: at
+// most item_max queries each, in bucket order; leafb = the leaf of every bucket
+// boundary.
+struct JoinItems {
+  Item *items = nullptr;
+  int64_t *n_items = nullptr;
+  const int32_t *leafb = nullptr;
+  uint32_t item_max = 0;
+};
+
 // ---- query pre-sort (partition.cu) ----
 // A batch set on the device: batches[b] holds queries [qpre[b], qpre[b+1])
 // of the set's concatenation (qpre has nb + 1 entries).
@@ -349,7 +370,7 @@ struct BatchView {
 // written to res1[place[i]] are in first-pass order, which
 // unpermute_first_pass takes back to the input order.
 int partition_queries_placed(const hm_tree *t, const int64_t *q, int64_t n, int bits, int64_t *q_out,
-                             int32_t *place, void *scratch, cudaStream_t s, const uint32_t **bucket_start,
+                             int32_t *place, void *scratch, cudaStream_t s, const JoinItems *ji,
                              const BatchView *bv = nullptr);
 int unpermute_first_pass(int64_t n, int bits, const int64_t *res1, int64_t *out, void *scratch, cudaStream_t s,
                          const BatchView *bv = nullptr);
@@ -358,13 +379,12 @@ int unpermute_first_pass(int64_t n, int bits, const int64_t *res1, int64_t *out,
 // unpermute_results (pos_out == nullptr); else it writes input positions.
 size_t partition_scratch_bytes(int64_t n, int bits, bool offsets, int batches = 1);  // batches: of a batch set
 // Groups queries by the top `bits` bits of their key (relative to the tree's
-// key range); *bucket_start (if given) receives a device pointer, inside the
-// scratch, to the 2^bits + 1 bucket starts.  pos_out: original position of
+// key range); ji (if given): the join's work items for the buckets.  pos_out: original position of
 // each grouped query (bits <= 8), or nullptr for the offset mode.
 // With bv, the queries are read from the batch set instead of q.
 int partition_queries(const hm_tree *t, const int64_t *q, int64_t n, int bits,
                       int64_t *q_out, int32_t *pos_out, void *scratch, cudaStream_t s,
-                      const uint32_t **bucket_start = nullptr, const BatchView *bv = nullptr);
+                      const JoinItems *ji = nullptr, const BatchView *bv = nullptr);
 // Offset mode: out[i] = result of input query i, given the results in grouped
 // order (res_sorted, clobbered) and the scratch of the matching partition.
 // With bv, the results go to the batch set's outputs instead of out.
@@ -407,10 +427,13 @@ void prof_end(hm_tree *t, int stage, int token, cudaStream_t s);
 int join_bits(const hm_tree *t);   // bucket bits for the join (leaves per bucket fit shared memory)
 bool join_fits(const hm_tree *t);  // the join supports this leaf size and its buckets fit on average
 size_t join_scratch_bytes(int64_t n, int bits);
+// Before the pre-sort: the bucket boundaries' leaves, and where the pre-sort
+// writes the items (scratch of join_scratch_bytes).
+int prepare_join(const hm_tree *t, int bits, int64_t n, void *scratch, cudaStream_t s, JoinItems *ji);
 // place: nullptr = results in grouped order (out[i] for grouped query i);
 // else out[place[i]].
-int launch_join(const hm_tree *t, const int64_t *qs, const uint32_t *bstart, int bits, int64_t n, int64_t *out,
-                void *scratch, cudaStream_t s, const int32_t *place = nullptr);
+int launch_join(const hm_tree *t, const int64_t *qs, int bits, int64_t n, int64_t *out, const JoinItems &ji,
+                cudaStream_t s, const int32_t *place = nullptr);
 
 // Opts kernel fn in to at least `bytes` of dynamic shared memory (and the
 // largest shared-memory carveout) on the current device, from any thread.

@@ -10,8 +10,8 @@
 // 31-bit images of their first keys (join_tma_kernel); 64-key leaves, and
 // batches of many queries per bucket, which first build a 64-slot directory of
 // the bucket, by per-thread cp.async (join_kernel).  The leaf range of each
-// bucket comes from one descent per bucket boundary (a separate kernel, one
-// thread per boundary; kept per tree shape between calls).  Leaves are read once
+// bucket comes from one descent per bucket boundary (a separate kernel; kept per
+// tree shape between calls).  Leaves are read once
 // per run and sequentially, so the DRAM traffic of a batch with more queries than
 // leaves falls from a random 160 B per query to the size of the touched leaf
 // region.  A bucket whose leaves do not fit shared memory (very skewed keys)
@@ -26,6 +26,7 @@
 // range whose first key is <= q is the leaf the descent would reach.
 #include "hm_internal.cuh"
 #include "async_copy.cuh"
+#include "warp_descent.cuh"
 
 #include <cuda.h>  // CUtensorMap and its enums; the encoder is fetched through the runtime
 
@@ -68,85 +69,23 @@ constexpr int kStageMax = (216 / kStages) * 1024;  // shared memory of one stage
 #endif
 static_assert(HM_JOIN_MAX_BITS <= 16, "a bucket number is kept in 16 bits");
 
-// A work item: some queries of one bucket, grouped queries
-// [qa, qa + len), and the bucket's leaves [l0, l0 + nl); the leaves are
-// staged once for all of them.
-struct __align__(16) Item {
-  int32_t qa, l0, b;  // first query, first leaf, bucket
-  uint32_t len_nl;    // queries << 16 | leaves (capped at 65535)
-  __host__ __device__ int len() const { return (int)(len_nl >> 16); }
-  __host__ __device__ int nl() const { return (int)(len_nl & 0xffffu); }
-};
-
 // leafb[b], b in [0, nb] = leaf holding the smallest key of bucket b (bucket
 // b's keys lie in leaves [leafb[b], leafb[b+1]]).  It depends only on the
 // inner nodes, the key range and the bucket bits, so the launcher keeps it
 // per tree shape and skips the descents while that holds.
+// A chain of dependent loads per boundary bounds it: a warp takes 32
+// neighbouring boundaries, which share most of their path, and ranks a node's
+// keys over its lanes (2^14 boundaries over 2^21 leaves: 7 us; one thread
+// each 15).
 __global__ void bucket_bounds_kernel(DevTree t, int f, int64_t lo, int shift, int nb, int32_t *__restrict__ leafb) {
   pdl_enter();
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x) {
-    if (b == 0) {
-      leafb[0] = 0;
-      continue;
-    }
-    if (b == nb) {
-      leafb[nb] = t.n_leaf - 1;
-      continue;
-    }
-    const uint64_t off = (uint64_t)b << shift;
-    if (off >= (uint64_t)kMaxKey - (uint64_t)lo) {  // boundary at or past Max_Key: no key above it
-      leafb[b] = t.n_leaf - 1;
-      continue;
-    }
-    leafb[b] = descend_leaf(t, f, (int64_t)((uint64_t)lo + off));
-  }
-}
-
-// The work items in bucket order and their number: CTA c owns buckets
-// [1024 c, 1024 c + 1024) and counts the items of those before them itself (at
-// most 64 loads a thread).
-constexpr int kItemThreads = 1024;
-
-__global__ void __launch_bounds__(kItemThreads) items_kernel(int nb, uint32_t item_max,
-                                                             const uint32_t *__restrict__ bstart,
-                                                             const int32_t *__restrict__ leafb,
-                                                             Item *__restrict__ items, int64_t *__restrict__ n_items) {
-  pdl_enter();
-  __shared__ uint32_t wsum[32], bsum[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int first = blockIdx.x * kItemThreads;
-  auto items_of = [&](int b) { return (bstart[b + 1] - bstart[b] + item_max - 1) / item_max; };
-  uint32_t before = 0;
-  for (int b = tid; b < first; b += kItemThreads) before += items_of(b);
-  const int b = first + tid;
-  const uint32_t mine = b < nb ? items_of(b) : 0;
-#pragma unroll
-  for (int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-  uint32_t incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) wsum[warp] = incl;
-  if (lane == 0) bsum[warp] = before;
-  __syncthreads();
-  uint32_t at = incl - mine;
-  for (int w = 0; w < 32; w++) at += bsum[w];
-  for (int w = 0; w < warp; w++) at += wsum[w];
-  if (b == nb - 1) *n_items = at + mine;
-  if (mine == 0) return;
-  const uint32_t s = bstart[b], e = bstart[b + 1];
-  const int32_t l0 = leafb[b], nl = leafb[b + 1] - l0 + 1;
-  for (uint32_t r = 0; r < mine; r++) {
-    const uint32_t qa = s + r * item_max;
-    Item it;
-    it.qa = (int32_t)qa;
-    it.l0 = l0;
-    it.b = b;
-    it.len_nl = min(item_max, e - qa) << 16 | (uint32_t)min(nl, 65535);  // a capped count is never staged
-    items[at + r] = it;
-  }
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if ((b & ~31) > nb) return;  // uniform in a warp
+  const uint64_t off = (uint64_t)min(b, nb) << shift;
+  // past the last boundary, and where it lies at or past Max_Key, no key is above it
+  const bool past = b >= nb || off >= (uint64_t)kMaxKey - (uint64_t)lo;
+  const int32_t leaf = descend_leaf_warp(t, f, past ? kMaxKey - 1 : (int64_t)((uint64_t)lo + off));
+  if (b <= nb) leafb[b] = b == 0 ? 0 : past ? t.n_leaf - 1 : leaf;
 }
 
 __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
@@ -658,8 +597,11 @@ int stage_leaves_for(const hm_tree *t, int bits) {
 
 int join_bits(const hm_tree *t) {
   // HM_JOIN_MAX_BITS bits, or fewer while buckets still average at most 32 leaves
+  // (64-key leaves: 16, with which more CTAs share an SM: 120 against 136 us for
+  // 6 M Zipf queries; 8: 157)
   int b = 1;
-  while (b < HM_JOIN_MAX_BITS && (t->n_leaf >> b) > 32) b++;
+  const int64_t most = t->cfg.leaf_cap == 16 ? 32 : 16;
+  while (b < HM_JOIN_MAX_BITS && (t->n_leaf >> b) > most) b++;
   return b;
 }
 
@@ -834,8 +776,10 @@ int run_tma_join(const hm_tree *t, TmaJoinKernel k, const CUtensorMap &tmap, int
   const unsigned grid = (unsigned)std::min<int64_t>(n_items_max, (int64_t)t->num_sms * per_sm);
   int rc = opt_in_smem((const void *)k, (int)kTmaSmem);
   if (rc) return rc;
-  launch_pdl(k, grid, kJoinThreads + 32, smem, s, tmap, t->view(), t->cfg.fanout, items, nitems, qs, place, out, ml,
-             biased(t->key_min), shift, t->d_err);
+  // not a dependent launch: CTAs that start behind the pre-sort's find an SM's
+  // shared memory carved out for those, and two of four fit (371 against 241 us)
+  k<<<grid, kJoinThreads + 32, smem, s>>>(tmap, t->view(), t->cfg.fanout, items, nitems, qs, place, out, ml,
+                                          biased(t->key_min), shift, t->d_err);
   note_launch();
   return HM_OK;
 }
@@ -848,8 +792,8 @@ int run_join(const hm_tree *t, JoinKernel k, int ml, int64_t n_items_max, const 
   const unsigned grid = (unsigned)std::min<int64_t>(n_items_max, (int64_t)t->num_sms * per_sm);
   int rc = opt_in_smem((const void *)k, kStages * kStageMax);
   if (rc) return rc;
-  launch_pdl(k, grid, kThreads, smem, s, t->view(), t->cfg.fanout, items, nitems, qs, place, out, ml,
-             biased(t->key_min), shift);
+  k<<<grid, kThreads, smem, s>>>(t->view(), t->cfg.fanout, items, nitems, qs, place, out, ml, biased(t->key_min),
+                                 shift);  // as above
   note_launch();
   return HM_OK;
 }
@@ -857,38 +801,60 @@ int run_join(const hm_tree *t, JoinKernel k, int ml, int64_t n_items_max, const 
 // measured: the directory pays from about three queries per thread and item
 bool use_dir(int64_t n, int nb) { return HM_JOIN_DIR_BITS > 0 && n >= (int64_t)HM_JOIN_DIR_MIN * nb; }
 
-}  // namespace
-
-int launch_join(const hm_tree *t, const int64_t *qs, const uint32_t *bstart, int bits, int64_t n, int64_t *out,
-                void *scratch, cudaStream_t s, const int32_t *place) {
-  if (n <= 0) return HM_OK;
-  const int nb = 1 << bits;
-  char *p = static_cast<char *>(scratch);
-  int32_t *leafb_s = reinterpret_cast<int32_t *>(p);
-  p += align_up(4 * (nb + 1), 256);
-  int64_t *n_items = reinterpret_cast<int64_t *>(p);
-  p += 256;
-  Item *items = reinterpret_cast<Item *>(p);
-  const int shift = bucket_shift(t, bits);
-  const int32_t *leafb = bucket_bounds(t, bits, shift, leafb_s, s);
-  const bool dir = use_dir(n, nb);
-  const JoinKernel k = place ? pick_join<true>(t->cfg.leaf_cap, dir) : pick_join<false>(t->cfg.leaf_cap, dir);
-  const int ml = stage_leaves_for(t, bits);
+// How the batch is joined: decided once, before its pre-sort.
+struct JoinChoice {
+  bool dir = false, tma = false;
+  int ml = 0, item_max = 0;
   CUtensorMap tmap;
-  const bool tma = HM_JOIN_TMA && !dir && tma_join_smem(ml) <= kTmaSmem && leaf_tensor_map(t, &tmap);
+};
+
+JoinChoice choose_join(const hm_tree *t, int bits, int64_t n) {
+  JoinChoice c;
+  c.dir = use_dir(n, 1 << bits);
+  c.ml = stage_leaves_for(t, bits);
+  c.tma = HM_JOIN_TMA && !c.dir && tma_join_smem(c.ml) <= kTmaSmem && leaf_tensor_map(t, &c.tmap);
   // the TMA join takes a step of queries per item: a fuller bucket's next step
   // is prefetched like any other item's
   const int64_t share = n / ((int64_t)t->num_sms * 16);
-  const int item_max = tma ? kJoinStep : (int)std::min<int64_t>(kItemMax, std::max<int64_t>(kItemMin, share / kRun * kRun));
-  launch_pdl(items_kernel, (unsigned)((nb + kItemThreads - 1) / kItemThreads), kItemThreads, 0, s, nb,
-             (uint32_t)item_max, bstart, leafb, items, n_items);
-  note_launch();
-  const int64_t most = max_items(n, nb, item_max);
-  int rc = tma ? run_tma_join(t, place ? pick_tma_join<true>(ml) : pick_tma_join<false>(ml), tmap, ml, most, items,
-                              n_items, qs, place, out, shift, s)
-               : run_join(t, k, ml, most, items, n_items, qs, place, out, shift, s);
-  if (rc) return rc;
+  c.item_max = c.tma ? kJoinStep : (int)std::min<int64_t>(kItemMax, std::max<int64_t>(kItemMin, share / kRun * kRun));
+  return c;
+}
+
+JoinItems join_layout(int bits, void *scratch, int32_t **leafb_scratch) {
+  char *p = static_cast<char *>(scratch);
+  *leafb_scratch = reinterpret_cast<int32_t *>(p);
+  p += align_up(4 * ((1 << bits) + 1), 256);
+  JoinItems ji;
+  ji.n_items = reinterpret_cast<int64_t *>(p);
+  ji.items = reinterpret_cast<Item *>(p + 256);
+  return ji;
+}
+
+}  // namespace
+
+int prepare_join(const hm_tree *t, int bits, int64_t n, void *scratch, cudaStream_t s, JoinItems *ji) {
+  int32_t *leafb_scratch = nullptr;
+  *ji = join_layout(bits, scratch, &leafb_scratch);
+  ji->leafb = bucket_bounds(t, bits, bucket_shift(t, bits), leafb_scratch, s);
+  ji->item_max = (uint32_t)choose_join(t, bits, n).item_max;
   return cuda_err(cudaGetLastError());
+}
+
+int launch_join(const hm_tree *t, const int64_t *qs, int bits, int64_t n, int64_t *out, const JoinItems &ji,
+                cudaStream_t s, const int32_t *place) {
+  if (n <= 0) return HM_OK;
+  const JoinChoice c = choose_join(t, bits, n);
+  const int shift = bucket_shift(t, bits);
+  const int64_t most = max_items(n, 1 << bits, c.item_max);
+  int rc;
+  if (c.tma) {
+    rc = run_tma_join(t, place ? pick_tma_join<true>(c.ml) : pick_tma_join<false>(c.ml), c.tmap, c.ml, most, ji.items,
+                      ji.n_items, qs, place, out, shift, s);
+  } else {
+    const JoinKernel k = place ? pick_join<true>(t->cfg.leaf_cap, c.dir) : pick_join<false>(t->cfg.leaf_cap, c.dir);
+    rc = run_join(t, k, c.ml, most, ji.items, ji.n_items, qs, place, out, shift, s);
+  }
+  return rc ? rc : cuda_err(cudaGetLastError());
 }
 
 }  // namespace hm

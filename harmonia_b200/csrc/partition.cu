@@ -1,7 +1,7 @@
 // Query pre-sort (the reference's PSA, "partially sorted aggregation"):
 // group a batch of queries by the top `bits` bits of their key, relative to
-// the tree's key range, report where each bucket starts, and afterwards move
-// per-query results from the grouped order back to the caller's order.
+// the tree's key range, cut the buckets into work items for the join, and
+// afterwards move per-query results from the grouped order back to the caller's order.
 //
 // The reference runs cub::DeviceRadixSort::SortPairs on bits [48,64) of
 // (key, pos) before every search launch
@@ -168,40 +168,89 @@ __global__ void __launch_bounds__(kCountThreads) psa_count_kernel(const int64_t 
 
 constexpr int kStartThreads = 1024;
 
-// Bucket starts (nb + 1) and the passes' cursors: CTA c owns buckets
-// [1024 c, 1024 c + 1024) and adds up the counts before them itself (at most
-// 64 loads a thread from L2).
+// Bucket starts (nb + 1), the passes' cursors and the join's work items: CTA c
+// owns buckets [1024 c, 1024 c + 1024) and adds up the counts and the items of
+// those before them itself (at most 64 loads a thread from L2); its items are
+// written a thread each, for a hot bucket has hundreds.  Launch latency and the
+// reload of the counts bound it: 13.6 us for 2^14 buckets, against 5.9 and
+// 10..17 us of two kernels.
 __global__ void __launch_bounds__(kStartThreads) psa_starts_kernel(const uint32_t *__restrict__ count, uint32_t nb,
                                                                    int l2, uint32_t n, uint32_t *__restrict__ start,
                                                                    uint32_t *__restrict__ cur1,
-                                                                   uint32_t *__restrict__ cur2) {
+                                                                   uint32_t *__restrict__ cur2, JoinItems ji) {
   pdl_enter();
-  __shared__ uint32_t wsum[32], bsum[32];
+  __shared__ uint32_t wsum[32], bsum[32], iwsum[32], ibsum[32];
+  __shared__ uint32_t upto[kStartThreads], from[kStartThreads], len[kStartThreads];  // items up to, start, count
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t first = blockIdx.x * kStartThreads;
-  uint32_t before = 0;
-  for (uint32_t i = tid; i < first; i += kStartThreads) before += count[i];
-  const uint32_t mine = first + tid < nb ? count[first + tid] : 0;
+  const uint32_t first = blockIdx.x * kStartThreads, im = ji.item_max;
+  auto items_of = [&](uint32_t c) { return im ? (c + im - 1) / im : 0; };
+  uint32_t before = 0, ibefore = 0;
+#pragma unroll 4
+  for (uint32_t i = tid; i < first; i += kStartThreads) {
+    const uint32_t c = count[i];
+    before += c;
+    ibefore += items_of(c);
+  }
+  const uint32_t mine = first + tid < nb ? count[first + tid] : 0, imine = items_of(mine);
 #pragma unroll
-  for (int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-  uint32_t incl = mine;
+  for (int o = 16; o; o >>= 1) {
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+    ibefore += __shfl_xor_sync(0xffffffffu, ibefore, o);
+  }
+  uint32_t incl = mine, iincl = imine;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o), z = __shfl_up_sync(0xffffffffu, iincl, o);
+    if (lane >= o) {
+      incl += y;
+      iincl += z;
+    }
   }
-  if (lane == 31) wsum[warp] = incl;
-  if (lane == 0) bsum[warp] = before;
+  if (lane == 31) {
+    wsum[warp] = incl;
+    iwsum[warp] = iincl;
+  }
+  if (lane == 0) {
+    bsum[warp] = before;
+    ibsum[warp] = ibefore;
+  }
   __syncthreads();
-  uint32_t at = incl - mine;
-  for (int w = 0; w < 32; w++) at += bsum[w];
-  for (int w = 0; w < warp; w++) at += wsum[w];
+  uint32_t at = incl - mine, iat = 0;
+  for (int w = 0; w < 32; w++) {
+    at += bsum[w];
+    iat += ibsum[w];
+  }
+  for (int w = 0; w < warp; w++) {
+    at += wsum[w];
+    iincl += iwsum[w];
+  }
   const uint32_t b = first + tid;
   if (b < nb) {
     start[b] = at;
     cur2[b] = at;
     if ((b & ((1u << l2) - 1)) == 0) cur1[b >> l2] = at;
     if (b == nb - 1) start[nb] = n;
+  }
+  if (im == 0) return;
+  upto[tid] = iincl;
+  from[tid] = at;
+  len[tid] = mine;
+  __syncthreads();
+  const uint32_t total = upto[kStartThreads - 1];
+  if (tid == 0 && first + kStartThreads >= nb) *ji.n_items = (int64_t)iat + total;
+  for (uint32_t x = tid; x < total; x += kStartThreads) {
+    uint32_t lo = 0;  // the bucket of item x: the first with upto > x
+#pragma unroll
+    for (uint32_t step = kStartThreads / 2; step > 0; step >>= 1)
+      if (upto[lo + step - 1] <= x) lo += step;
+    const uint32_t done = (x - (lo ? upto[lo - 1] : 0)) * im;
+    const int32_t l0 = ji.leafb[first + lo], nl = ji.leafb[first + lo + 1] - l0 + 1;
+    Item it;
+    it.qa = (int32_t)(from[lo] + done);
+    it.l0 = l0;
+    it.b = (int32_t)(first + lo);
+    it.len_nl = min(im, len[lo] - done) << 16 | (uint32_t)min(nl, 65535);  // a capped count is never staged
+    ji.items[iat + x] = it;
   }
 }
 
@@ -525,7 +574,7 @@ size_t work_layout(int64_t n, int bits, bool offsets, Work *w, char *base, int b
 
 // Counts, starts and (batch sets) the first pass's tiles.
 void count_and_start(const Work &w, const Bucket &bk, const int64_t *q, int64_t n, int bits, int sms, cudaStream_t s,
-                     const BatchView *bv) {
+                     const JoinItems *ji, const BatchView *bv) {
   const uint32_t nb = 1u << bits;
   cudaMemsetAsync(w.count, 0, 4 * (size_t)nb, s);
   const size_t smem = ((size_t)nb * 2 + 15) & ~(size_t)15;
@@ -544,7 +593,8 @@ void count_and_start(const Work &w, const Bucket &bk, const int64_t *q, int64_t 
   }
   const int l2 = bits > 8 ? bits - 8 : 0;
   launch_pdl(psa_starts_kernel, (nb + kStartThreads - 1) / kStartThreads, kStartThreads, 0, s,
-             static_cast<const uint32_t *>(w.count), nb, l2, (uint32_t)n, w.start, w.cur1, w.cur2);
+             static_cast<const uint32_t *>(w.count), nb, l2, (uint32_t)n, w.start, w.cur1, w.cur2,
+             ji ? *ji : JoinItems());
   note_launch(bv ? 3 : 2);
 }
 
@@ -602,7 +652,7 @@ size_t partition_scratch_bytes(int64_t n, int bits, bool offsets, int batches) {
 }
 
 int partition_queries(const hm_tree *t, const int64_t *q, int64_t n, int bits, int64_t *q_out, int32_t *pos_out,
-                      void *scratch, cudaStream_t s, const uint32_t **bucket_start, const BatchView *bv) {
+                      void *scratch, cudaStream_t s, const JoinItems *ji, const BatchView *bv) {
   if (n == 0) return HM_OK;
   if (bits < 1 || bits > 16 || n > INT32_MAX || n < 0) return HM_EINVAL;
   const bool offsets = pos_out == nullptr;
@@ -610,7 +660,7 @@ int partition_queries(const hm_tree *t, const int64_t *q, int64_t n, int bits, i
   Work w;
   work_layout(n, bits, offsets, &w, static_cast<char *>(scratch), bv ? bv->nb : 1);
   const Bucket bk = make_bucket(t, bits);
-  count_and_start(w, bk, q, n, bits, t->num_sms, s, bv);
+  count_and_start(w, bk, q, n, bits, t->num_sms, s, ji, bv);
   if (!offsets) {
     one_pass<int32_t, false, false, kSmallThreads, kSmallPer, kSmallCtas>(w, bk, q, n, bits, w.cur1, q_out, pos_out,
                                                                           nullptr, s);
@@ -620,23 +670,21 @@ int partition_queries(const hm_tree *t, const int64_t *q, int64_t n, int bits, i
     first_pass(w, bk, q, n, bits, w.q_tmp, static_cast<uint16_t *>(w.pay1), s, bv);
     one_pass<uint16_t, true>(w, bk, w.q_tmp, n, bits, w.cur2, q_out, w.loc, &w.p2, s);
   }
-  if (bucket_start) *bucket_start = w.start;
   return cuda_err(cudaGetLastError());
 }
 
 int partition_queries_placed(const hm_tree *t, const int64_t *q, int64_t n, int bits, int64_t *q_out,
-                             int32_t *place, void *scratch, cudaStream_t s, const uint32_t **bucket_start,
+                             int32_t *place, void *scratch, cudaStream_t s, const JoinItems *ji,
                              const BatchView *bv) {
   if (n == 0) return HM_OK;
   if (bits <= 8 || bits > 16 || n > INT32_MAX || n < 0 || !place) return HM_EINVAL;
   Work w;
   work_layout(n, bits, true, &w, static_cast<char *>(scratch), bv ? bv->nb : 1);
   const Bucket bk = make_bucket(t, bits);
-  count_and_start(w, bk, q, n, bits, t->num_sms, s, bv);
+  count_and_start(w, bk, q, n, bits, t->num_sms, s, ji, bv);
   first_pass(w, bk, q, n, bits, w.q_tmp, static_cast<uint16_t *>(w.pay1), s, bv);
   one_pass<int32_t, true, false, kSmallThreads, kSmallPer, kSmallCtas>(w, bk, w.q_tmp, n, bits, w.cur2, q_out, place,
                                                                        nullptr, s);
-  if (bucket_start) *bucket_start = w.start;
   return cuda_err(cudaGetLastError());
 }
 
