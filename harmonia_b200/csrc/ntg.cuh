@@ -35,6 +35,17 @@ __device__ __forceinline__ longlong2 ldg2(const int64_t *p, uint64_t pol) {
                : "l"(p), "l"(pol));
   return r;
 }
+// 32-B read-only global load with an L2 cache policy; p 32-byte aligned.
+struct Quad {
+  int64_t x[4];
+};
+__device__ __forceinline__ Quad ldg4(const int64_t *p, uint64_t pol) {
+  Quad r;
+  asm volatile("ld.global.nc.L2::cache_hint.v4.b64 {%0, %1, %2, %3}, [%4], %5;"
+               : "=l"(r.x[0]), "=l"(r.x[1]), "=l"(r.x[2]), "=l"(r.x[3])
+               : "l"(p), "l"(pol));
+  return r;
+}
 __device__ __forceinline__ int64_t ldg1(const int64_t *p, uint64_t pol) {
   int64_t r;
   asm volatile("ld.global.nc.L2::cache_hint.s64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(pol));
@@ -67,6 +78,16 @@ __device__ __forceinline__ int group_sum(int v) {
 // group (lane `sub` reads vectors sub, sub+W, ...).
 template <int W, int LEN, bool SMEM>
 __device__ __forceinline__ int count_le(const int64_t *p, int64_t q, int sub, uint64_t pol) {
+  if constexpr (!SMEM && LEN % (4 * W) == 0) {  // rows are 32-byte aligned; half the requests of 16-B loads
+    constexpr int N = LEN / (4 * W);
+    Quad v[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) v[i] = ldg4(p + 4 * (sub + i * W), pol);
+    int c = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) c += (v[i].x[0] <= q) + (v[i].x[1] <= q) + (v[i].x[2] <= q) + (v[i].x[3] <= q);
+    return group_sum<W>(c);
+  }
   constexpr int NV = LEN / 2;
   constexpr int VPL = (NV + W - 1) / W;
   longlong2 v[VPL];

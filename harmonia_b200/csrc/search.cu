@@ -84,6 +84,11 @@ __device__ __forceinline__ int match_slot(const int64_t *p, int64_t q, int sub, 
 // 2^26 keys: 18.2 Gq/s at one query per group against 15.4 for the best
 // setting without it; at two queries per group the extra registers cost more
 // than the round trip saves (12.6), so only Q = 1 uses it.
+// What bounds a batch of many tiles is the L1 data pipe (87 % of its peak rate
+// of wavefronts, L2 37 %, DRAM 43 % for 2^20 queries of 2^24 keys): a wavefront
+// per line that a request touches.  With 32 bytes a lane one request covers a
+// group's 128-B line, half as many wavefronts at the leaf (2^20 queries: 60.6 ->
+// 55.6 us at 2^24 keys, 70.7 -> 66.0 at 2^26).  Wider groups would leave lanes idle.
 #ifndef HM_LEAF_VALUES_WITH_KEYS
 #define HM_LEAF_VALUES_WITH_KEYS 1
 #endif
@@ -91,6 +96,23 @@ template <int W, int LC>
 __device__ __forceinline__ int64_t match_value(const int64_t *p, int64_t q, int sub, uint64_t pol, bool *hit) {
   constexpr int NV = LC / 2;
   constexpr int VPL = (NV + W - 1) / W;
+  if constexpr (W <= 4) {  // a 128-B line of keys takes W lanes 4 / W loads
+    Quad v[VPL / 2], w[VPL / 2];
+#pragma unroll
+    for (int i = 0; i < VPL / 2; i++) {
+      v[i] = ldg4(p + 4 * (sub + i * W), pol);
+      w[i] = ldg4(p + LC + 4 * (sub + i * W), pol);
+    }
+    int64_t r = HM_NOT_FOUND;
+    bool h = false;
+#pragma unroll
+    for (int i = 0; i < VPL / 2; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (v[i].x[j] == q) { r = w[i].x[j]; h = true; }
+    *hit = h;
+    return r;
+  }
   longlong2 v[VPL], w[VPL];
 #pragma unroll
   for (int i = 0; i < VPL; i++) {
