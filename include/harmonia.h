@@ -85,7 +85,8 @@ typedef struct {
   int queries_per_group; /* queries a group keeps in flight: 1,2,4 (default 1; at 1 a 16-key leaf's
                             values load with its keys) */
   int sort_bits;         /* query pre-sort: top bits, 0 = off, 1..16, -1 = auto (default -1) */
-  int smem_bytes;        /* budget for top levels staged in shared memory (default 49152) */
+  int smem_bytes;        /* budget for top levels staged in shared memory (default 49152;
+                         * up to that, levels are staged while they fit 16384) */
   int cache_hints;       /* L2 policy: 1 = inner rows evict_last, leaves evict_first; 2 = none
                             (default 1) */
   int join;              /* large batches: 1 = pre-sort + bucket join, 2 = never, -1 = when the
