@@ -358,7 +358,10 @@ __global__ void __launch_bounds__(kThreads, HM_JOIN_MINB) join_kernel(DevTree t,
 // bound), the slot by four probes of the leaf's keys whose swizzled address is
 // one exclusive-or.  Two first keys with one image make the search end on a
 // leaf past the key's, seen by its first key being above the key, and step
-// back.  kJoinStep covers a bucket of 256 queries and four standard deviations.  An item takes one CTA barrier: past it every thread
+// back.  Leaves and queries past the bucket take the last image, so the step
+// back decides between them too: a replayed plan keeps the buckets of its
+// capture, while write epochs may since have put larger keys into the last
+// leaves.  kJoinStep covers a bucket of 256 queries and four standard deviations.  An item takes one CTA barrier: past it every thread
 // has left the item before, whose stage is then filled again.
 // 2^24 queries on 2^26 keys (1.41 GB of records, queries, places and results):
 // 241 us, 5.9 TB/s, 0.90 of the measured copy rate.  Before, with one thread
@@ -485,7 +488,7 @@ __global__ void __launch_bounds__(kJoinThreads + 32, kJoinCtas) join_tma_kernel(
           if (m < nl) {
             const uint64_t k = biased(lds64(kb + m * 128 + ((m & 7) << 4)));
             const uint64_t d = k <= lo_u ? 0 : (k - lo_u) >> ishift;
-            v = d > kImageMax ? kImageMax + 1 : (uint32_t)d;  // a leaf past the bucket
+            v = (uint32_t)min(d, (uint64_t)kImageMax);
           }
           asm volatile("st.shared.u32 [%0], %1;" ::"r"(im + m * 4), "r"(v) : "memory");
         }
