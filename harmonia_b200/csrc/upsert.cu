@@ -92,59 +92,105 @@ __global__ void lsd_finish_kernel(const uint64_t *__restrict__ uk, int64_t n, in
 // Ctl::user of an epoch.
 enum { kUserChanged = 0, kUserOverflow = 1, kUserEmpty = 2, kUserErr = 3 };  // keys added or removed; ...; error word
 
-// Whether a set bit of mask before position i belongs to a key of the same
-// leaf as position i's.  (A leaf's keys are one run of the sorted batch.)
-__device__ __forceinline__ bool marked_before(const uint32_t *__restrict__ mask, const int32_t *__restrict__ leaf_of,
-                                              int64_t i, int32_t leaf) {
-  while (i > 0 && leaf_of[i - 1] == leaf) {
-    const int64_t w = (i - 1) >> 5;
-    const uint32_t m = mask[w] & (0xffffffffu >> (31 - ((i - 1) & 31)));
-    if (m) return leaf_of[w * 32 + 31 - __clz(m)] == leaf;
-    i = w * 32;
+// A leaf's keys are one run of the sorted batch.  Nearly all runs end within a
+// word of the mask, but a key that fills much of a batch makes a long one, of
+// which few keys or none are marked.  A warp looks through such a run's marks
+// kMarkStep words at a time, a latency of memory each, in a function of its own.
+// 4096K keys, half of them one new key: 0.78 ms, 33.9 with a word at a time
+// (0.66 without the new key).
+constexpr int kMarkWords = 16, kMarkStep = 32 * kMarkWords;
+
+// The nearest word with a set bit in a step of the mask: words w0 + d, w0 + 2 d,
+// ... (d = 1 or -1) as far as they are in [0, words); -1 if none (all lanes).
+__device__ __forceinline__ int64_t marked_word(const uint32_t *__restrict__ mask, int64_t w0, int d, int64_t words,
+                                               uint32_t *bits) {
+  const int lane = threadIdx.x & 31;
+  uint32_t v[kMarkWords], any = 0;
+#pragma unroll
+  for (int x = 0; x < kMarkWords; x++) {
+    const int64_t at = w0 + d * (x * 32 + lane + 1);
+    v[x] = at >= 0 && at < words ? mask[at] : 0;
+  }
+#pragma unroll
+  for (int x = 0; x < kMarkWords; x++) any |= v[x];
+  if (!__any_sync(0xffffffffu, any != 0)) return -1;
+  int64_t found = -1;
+#pragma unroll
+  for (int x = 0; x < kMarkWords; x++) {
+    const uint32_t some = __ballot_sync(0xffffffffu, v[x] != 0);
+    if (some && found < 0) {
+      const int from = __ffs(some) - 1;
+      *bits = __shfl_sync(0xffffffffu, v[x], from);
+      found = w0 + d * (x * 32 + from + 1);
+    }
+  }
+  return found;
+}
+
+// The rest of marked_before from word w on, and of next_marked.
+__device__ __noinline__ bool marked_before_word(const uint32_t *__restrict__ mask, const int32_t *__restrict__ leaf_of,
+                                                int64_t w, int64_t words, int32_t leaf) {
+  for (; w > 0 && leaf_of[w * 32 - 1] == leaf; w -= kMarkStep) {
+    uint32_t bits = 0;
+    const int64_t at = marked_word(mask, w, -1, words, &bits);
+    if (at >= 0) return leaf_of[at * 32 + 31 - __clz(bits)] == leaf;
   }
   return false;
 }
-
-// First set bit of mask at or after i whose key lies in `leaf`; -1 if none.
-__device__ __forceinline__ int64_t next_marked(const uint32_t *__restrict__ mask, const int32_t *__restrict__ leaf_of,
-                                               int64_t i, int64_t n, int32_t leaf) {
-  while (i < n && leaf_of[i] == leaf) {
-    const uint32_t m = mask[i >> 5] >> (i & 31);
-    if (m) {
-      i += __ffs(m) - 1;
+__device__ __noinline__ int64_t marked_from_word(const uint32_t *__restrict__ mask, const int32_t *__restrict__ leaf_of,
+                                                 int64_t w, int64_t words, int32_t leaf) {
+  for (; w < words && leaf_of[w * 32] == leaf; w += kMarkStep) {
+    uint32_t bits = 0;
+    const int64_t at = marked_word(mask, w - 1, 1, words, &bits);
+    if (at >= 0) {
+      const int64_t i = at * 32 + __ffs(bits) - 1;
       return leaf_of[i] == leaf ? i : -1;
     }
-    i = (i | 31) + 1;
   }
   return -1;
 }
 
-// Up to 32 marked keys of the sorted batch that a warp works on.
-struct WarpRows {
-  int64_t key[32], val[32];  // by lane (upsert)
-  uint32_t members[32];      // the lanes of the r-th leaf
-  int32_t head[32];          // the first of them
-};
+// Whether a set bit of mask before position i belongs to a key of the same
+// leaf as position i's (all lanes, the same arguments).
+__device__ __forceinline__ bool marked_before(const uint32_t *__restrict__ mask, const int32_t *__restrict__ leaf_of,
+                                              int64_t i, int64_t n, int32_t leaf) {
+  if (i == 0 || leaf_of[i - 1] != leaf) return false;
+  const int64_t w = (i - 1) >> 5;
+  const uint32_t m = mask[w] & (0xffffffffu >> (31 - ((i - 1) & 31)));
+  if (m) return leaf_of[w * 32 + 31 - __clz(m)] == leaf;
+  return marked_before_word(mask, leaf_of, w, (n + 31) / 32, leaf);
+}
 
-// The last leaf's new keys past the warp's 32.
-struct NextKeys {
-  int32_t leaf = -1;  // the last leaf
-  int64_t at = 0;     // where its other keys may follow
-  const uint32_t *mask = nullptr;
-  const int32_t *leaf_of = nullptr;
-  const int64_t *sk = nullptr;
-  const int32_t *spos = nullptr;
-  const int64_t *vals = nullptr;
-  int64_t n = 0;
+// First set bit of mask at or after i whose key lies in `leaf`; -1 if none
+// (all lanes, the same arguments).
+__device__ __forceinline__ int64_t next_marked(const uint32_t *__restrict__ mask, const int32_t *__restrict__ leaf_of,
+                                               int64_t i, int64_t n, int32_t leaf) {
+  if (i >= n || leaf_of[i] != leaf) return -1;
+  const uint32_t m = mask[i >> 5] >> (i & 31);
+  if (m) {
+    i += __ffs(m) - 1;
+    return leaf_of[i] == leaf ? i : -1;
+  }
+  return marked_from_word(mask, leaf_of, (i >> 5) + 1, (n + 31) / 32, leaf);
+}
+
+// Up to 32 marked keys of the sorted batch that a warp works on, and the last
+// leaf's marked keys past them (one more than it can hold at most).
+template <int LC>
+struct WarpRows {
+  int64_t key[32 + LC + 1], val[32 + LC + 1];  // by lane, then the last leaf's others (upsert)
+  uint32_t members[32];                        // the lanes of the r-th leaf
+  int32_t head[32];                            // the first of them
 };
 
 // The rows of the nh listed leaves, by groups of LC / 4 lanes that hold four
 // slots each (eight 16-key leaves at a time).  Upsert: a leaf's new keys are
 // placed among the sorted ones; a leaf without room for all of them is left as
 // it is.  Delete: the emptied slots (Max_Key) are squeezed out in key order.
-// Adds the keys stored or removed to *changed (per lane).
+// Adds the keys stored or removed to *changed (per lane).  The leaf `last` has
+// `extra` keys past the warp's 32.
 template <int LC, bool DEL>
-__device__ __forceinline__ void write_rows(WarpRows &wr, int nh, int32_t leaf, const NextKeys &nx,
+__device__ __forceinline__ void write_rows(WarpRows<LC> &wr, int nh, int32_t leaf, int32_t last, int extra,
                                            int64_t *leaf_rows, int32_t *leaf_cnt, bsort::Ctl *ctl, int *changed) {
   constexpr int LI = LC >= 32 ? LC / 8 : 0;
   constexpr int ROW = LI + 2 * LC;
@@ -215,29 +261,28 @@ __device__ __forceinline__ void write_rows(WarpRows &wr, int nh, int32_t leaf, c
         to[x] = 4 * g + x;
         ns[x] = -1;
       }
-      bool on = act && lf == nx.leaf, over = false;  // its run may go on
-      int64_t at = nx.at;
-      while (__any_sync(0xffffffffu, todo != 0 || on)) {
+      int more = act && lf == last ? extra : 0, at = 32;
+      bool over = false;
+      while (__any_sync(0xffffffffu, todo != 0 || more > 0)) {
         int64_t q = 0, val = 0;
-        bool have = todo != 0;
+        bool have = todo != 0 || more > 0;
         if (have) {
-          const int j = __ffs(todo) - 1;
-          todo &= todo - 1;
+          int j = at;
+          if (todo != 0) {
+            j = __ffs(todo) - 1;
+            todo &= todo - 1;
+          } else {
+            at++;
+            more--;
+          }
           q = wr.key[j];
           val = wr.val[j];
-        } else if (on) {
-          at = next_marked(nx.mask, nx.leaf_of, at, nx.n, lf);
-          on = have = at >= 0;
-          if (have) {
-            q = nx.sk[at];
-            val = nx.vals[nx.spos[at]];
-            at++;
-          }
         }
         if (have && cnt + m == LC) {  // no room
           over = true;
-          have = on = false;
+          have = false;
           todo = 0;
+          more = 0;
         }
         int below = 0;
 #pragma unroll
@@ -408,19 +453,21 @@ __device__ __forceinline__ int nth_bit(uint32_t w, int k) {
 // The rows of the leaves of the marked keys.  A warp takes wpw words of the
 // mask (few in a small batch, for more warps) and their marked keys 32 at a
 // time, one per lane, so that their loads are in flight together; a leaf is
-// handled where its first marked key lies.
+// handled where its first marked key lies.  The bounds hold the registers at
+// what the short runs need: with 80 instead of 72 the epoch pair of 4096K keys
+// takes 544 instead of 536 us.
 template <int LC, bool DEL>
-__global__ void __launch_bounds__(kRowThreads) leaf_rows_kernel(const int64_t *__restrict__ sk,
+__global__ void __launch_bounds__(kRowThreads, DEL ? 10 : 7) leaf_rows_kernel(const int64_t *__restrict__ sk,
                                                                 const int32_t *__restrict__ spos,
                                                                 const int64_t *__restrict__ vals, int64_t n, int wpw,
                                                                 const int32_t *__restrict__ leaf_of,
                                                                 const uint32_t *__restrict__ mask, int64_t *leaf_rows,
                                                                 int32_t *leaf_cnt, bsort::Ctl *ctl) {
   pdl_enter();
-  __shared__ WarpRows s_rows[kRowThreads / 32];
+  __shared__ WarpRows<LC> s_rows[kRowThreads / 32];
   if (ctl->skew || (!DEL && (ctl->flags & 2u))) return;
   const int lane = threadIdx.x & 31;
-  WarpRows &wr = s_rows[threadIdx.x >> 5];
+  WarpRows<LC> &wr = s_rows[threadIdx.x >> 5];
   const int64_t words = (n + 31) / 32;
   const int64_t base = (blockIdx.x * (int64_t)(kRowThreads / 32) + (threadIdx.x >> 5)) * wpw;
   const uint32_t mine = lane < wpw && base + lane < words ? mask[base + lane] : 0;
@@ -451,7 +498,10 @@ __global__ void __launch_bounds__(kRowThreads) leaf_rows_kernel(const int64_t *_
     }
     const int32_t up = __shfl_up_sync(0xffffffffu, leaf, 1);
     bool head = valid && leaf != (lane == 0 ? last : up);
-    if (c0 == 0 && lane == 0) head = !marked_before(mask, leaf_of, i, leaf);
+    if (c0 == 0) {
+      const bool before = marked_before(mask, leaf_of, __shfl_sync(0xffffffffu, i, 0), n, __shfl_sync(0xffffffffu, leaf, 0));
+      if (lane == 0) head = !before;
+    }
     const uint32_t heads = __ballot_sync(0xffffffffu, head);
     const uint32_t members = __match_any_sync(0xffffffffu, leaf) & __ballot_sync(0xffffffffu, valid);
     if (head) {
@@ -460,10 +510,20 @@ __global__ void __launch_bounds__(kRowThreads) leaf_rows_kernel(const int64_t *_
       wr.members[h] = members;
     }
     last = __shfl_sync(0xffffffffu, leaf, 31);
-    NextKeys nx;
-    if (!DEL) nx = NextKeys{last, __shfl_sync(0xffffffffu, i, 31) + 1, mask, leaf_of, sk, spos, vals, n};
+    int extra = 0;
+    if (!DEL) {
+      for (int64_t at = __shfl_sync(0xffffffffu, i, 31) + 1; extra <= LC; at++) {
+        at = next_marked(mask, leaf_of, at, n, last);
+        if (at < 0) break;
+        if (lane == 0) {
+          wr.key[32 + extra] = sk[at];
+          wr.val[32 + extra] = vals[spos[at]];
+        }
+        extra++;
+      }
+    }
     __syncwarp();
-    write_rows<LC, DEL>(wr, __popc(heads), leaf, nx, leaf_rows, leaf_cnt, ctl, &changed);
+    write_rows<LC, DEL>(wr, __popc(heads), leaf, last, extra, leaf_rows, leaf_cnt, ctl, &changed);
   }
   changed = __reduce_add_sync(0xffffffffu, changed);
   if (lane == 0 && changed > 0) atomicAdd(&ctl->user[kUserChanged], (unsigned long long)changed);
