@@ -49,15 +49,18 @@ constexpr int kSmallThreads = 512, kSmallPer = 8, kSmallCtas = 3;
 constexpr int kSmallTile = kSmallThreads * kSmallPer;
 static_assert(kTile < 65536 && kTileThreads >= 256 && kSmallThreads >= 256, "16-bit offsets; a thread per digit");
 
-// Bucket of a key: top `bits` bits of (k - lo) over the tree's key range.
+// Bucket of a key: top `bits` bits of (k - lo) over the tree's key range.  The
+// join finds a bucket's leaves from the same boundaries, so a key above the
+// range stays in the bucket of its offset while there is one: a replayed plan's
+// range is that of its capture, and the tree may hold larger keys by then.
 struct Bucket {
-  int64_t lo, hi;
+  int64_t lo;
   int shift;
   int maxd;
   __device__ __forceinline__ int operator()(int64_t k) const {
     if (k <= lo) return 0;
-    if (k >= hi) return maxd;
-    return (int)(((uint64_t)k - (uint64_t)lo) >> shift);
+    const uint64_t d = ((uint64_t)k - (uint64_t)lo) >> shift;
+    return d > (uint64_t)maxd ? maxd : (int)d;
   }
 };
 
@@ -509,7 +512,6 @@ __global__ void __launch_bounds__(kRevThreads, kRevCtas) psa_unpermute_kernel(
 Bucket make_bucket(const hm_tree *t, int bits) {
   Bucket d;
   d.lo = t->key_min;
-  d.hi = t->key_max;
   d.maxd = (1 << bits) - 1;
   uint64_t range = (uint64_t)t->key_max - (uint64_t)t->key_min;
   int len = 0;

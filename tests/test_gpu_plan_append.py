@@ -54,3 +54,27 @@ def test_keys_past_the_captured_end(span, how, n_q):
             torch.cuda.synchronize()
             assert (dout.cpu().numpy() == oracle.search(q)).all()
             assert (t.search(dq).cpu().numpy() == oracle.search(q)).all()
+
+
+@pytest.mark.parametrize("n_q", [20_000, 400_000])
+@pytest.mark.parametrize("leaf_cap,fill", [(16, 12), (64, 48)])
+def test_keys_between_the_captured_end_and_the_last_bucket(leaf_cap, fill, n_q):
+    # the captured range ends a little past the middle of the buckets
+    n = 1 << 17
+    sk = np.arange(n, dtype=np.int64) * (1 << 20) * 9 // 8
+    sv = dg.values_for(sk)
+    new = sk[-1] + np.arange(1, 15 * leaf_cap, dtype=np.int64) * (1 << 29)
+    q = np.concatenate([new, new + 1, sk[-40:], dg.gen_point_queries(sk, n_q, 0.9, seed=6)])
+    with BPlusTree.bulk_load(cuda(sk), cuda(sv), leaf_cap=leaf_cap, leaf_fill=fill) as t:
+        t.set_search_config(join=1)
+        dq, dout = cuda(q), torch.empty(len(q), dtype=torch.int64, device="cuda")
+        with t.plan([(dq, dout)]) as plan:
+            rows = t.info().leaf_rows
+            t.upsert(cuda(new), cuda(new - 5))
+            sk, sv = po.upsert_set(sk, sv, new, new - 5)
+            assert t.info().leaf_rows == rows  # no rebuild
+            oracle = po.PortTree(sk, sv)
+            plan.launch()
+            torch.cuda.synchronize()
+            assert (dout.cpu().numpy() == oracle.search(q)).all()
+            assert (t.search(dq).cpu().numpy() == oracle.search(q)).all()
