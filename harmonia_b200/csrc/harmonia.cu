@@ -164,30 +164,18 @@ std::mutex g_slot_mu;
 std::vector<char *> g_slots;        // free ones
 std::vector<void *> g_slot_chunks;  // the allocations
 
-char *take_slot() {
-  std::lock_guard<std::mutex> lk(g_slot_mu);
-  if (g_slots.empty()) {
-    void *p = nullptr;
-    if (cudaHostAlloc(&p, kSlot * kSlotChunk, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    g_slot_chunks.push_back(p);
-    for (int i = 0; i < kSlotChunk; i++) g_slots.push_back(static_cast<char *>(p) + i * kSlot);
-  }
-  char *c = g_slots.back();
-  g_slots.pop_back();
-  return c;
-}
-
-void give_slot(char *p) {
-  std::lock_guard<std::mutex> lk(g_slot_mu);
-  g_slots.push_back(p);
-}
+// Making a slot and waiting for it may meet a thread that captures another
+// stream: neither touches that stream, so neither is refused for it.
+struct OutsideCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 
 void trim_slots() {
   std::lock_guard<std::mutex> lk(g_slot_mu);
   if (g_slots.size() != g_slot_chunks.size() * kSlotChunk) return;
+  OutsideCapture guard;
   for (void *p : g_slot_chunks) cudaFreeHost(p);
   g_slot_chunks.clear();
   g_slots.clear();
@@ -200,20 +188,52 @@ __global__ void publish_kernel(uint32_t *host, const uint32_t *src, int words, c
 }
 }  // namespace
 
-int read_back(void *dst, const void *src, size_t bytes, cudaStream_t s, const unsigned *d_err, unsigned *err) {
-  char *slot = take_slot();
-  if (!slot) return HM_ENOMEM;
+ReadSlot::ReadSlot() {
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  if (g_slots.empty()) {
+    try {  // room for the list of all slots, so that giving one back needs no memory
+      g_slot_chunks.reserve(g_slot_chunks.size() + 1);
+      g_slots.reserve((g_slot_chunks.size() + 1) * kSlotChunk);
+    } catch (const std::bad_alloc &) {
+      return;
+    }
+    OutsideCapture guard;
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, kSlot * kSlotChunk, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    g_slot_chunks.push_back(p);
+    for (int i = 0; i < kSlotChunk; i++) g_slots.push_back(static_cast<char *>(p) + i * kSlot);
+  }
+  p_ = g_slots.back();
+  g_slots.pop_back();
+}
+
+ReadSlot::~ReadSlot() {
+  if (!p_) return;
+  std::lock_guard<std::mutex> lk(g_slot_mu);
+  g_slots.push_back(p_);
+}
+
+int ReadSlot::read(void *dst, const void *src, size_t bytes, cudaStream_t s, const unsigned *d_err,
+                   unsigned *err) const {
+  if (!p_) return HM_ENOMEM;
+  OutsideCapture guard;
   const int err_at = (int)(kReadBack / 4);
-  cudaError_t e = launch_pdl(publish_kernel, 1, 32, 0, s, reinterpret_cast<uint32_t *>(slot),
+  cudaError_t e = launch_pdl(publish_kernel, 1, 32, 0, s, reinterpret_cast<uint32_t *>(p_),
                              static_cast<const uint32_t *>(src), (int)(bytes / 4), d_err, err_at);
   note_launch();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) {
-    std::memcpy(dst, slot, bytes);
-    if (err) std::memcpy(err, slot + kReadBack, 4);
+    std::memcpy(dst, p_, bytes);
+    if (err) std::memcpy(err, p_ + kReadBack, 4);
   }
-  give_slot(slot);
   return cuda_err(e);
+}
+
+int read_back(void *dst, const void *src, size_t bytes, cudaStream_t s, const unsigned *d_err, unsigned *err) {
+  return ReadSlot().read(dst, src, bytes, s, d_err, err);
 }
 
 // Scratch blocks come from the block cache above and grow by half again when

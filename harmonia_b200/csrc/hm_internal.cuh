@@ -498,11 +498,27 @@ void dev_release(void *p);
 void release_after(void *p, cudaStream_t s);
 
 // ---- small results to the host (harmonia.cu) ----
-// Waits for stream s and brings `bytes` (at most kReadBack) of device memory at
-// src to dst and, if err is given, the word at d_err to *err.  A one-warp
-// kernel writes them to page-locked memory that the device maps, so the call
-// costs one wait and no copy through the driver's staging.
+// A page-locked slot that the device maps, for the time of a call.  read()
+// waits for stream s and brings `bytes` (at most kReadBack) of device memory at
+// src to dst and, if err is given, the word at d_err to *err: a one-warp kernel
+// writes them to the slot, so the call costs one wait and no copy through the
+// driver's staging.  A call that changes the tree takes its slot first: without
+// one (ok() is false, HM_ENOMEM) nothing may have been enqueued.
 constexpr size_t kReadBack = 192;
+class ReadSlot {
+ public:
+  ReadSlot();
+  ~ReadSlot();
+  ReadSlot(const ReadSlot &) = delete;
+  ReadSlot &operator=(const ReadSlot &) = delete;
+  bool ok() const { return p_ != nullptr; }
+  int read(void *dst, const void *src, size_t bytes, cudaStream_t s, const unsigned *d_err = nullptr,
+           unsigned *err = nullptr) const;
+
+ private:
+  char *p_ = nullptr;
+};
+// The same with a slot of its own.
 int read_back(void *dst, const void *src, size_t bytes, cudaStream_t s, const unsigned *d_err = nullptr,
               unsigned *err = nullptr);
 

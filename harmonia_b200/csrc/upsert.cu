@@ -754,6 +754,7 @@ struct Epoch {
   uint32_t *mask = nullptr;
   void *sort_scratch = nullptr, *scan_scratch = nullptr;
   bsort::Ctl *ctl = nullptr;
+  ReadSlot slot;  // held before the tree changes: its size and key range follow from what is read
 
   static size_t sort_bytes(int64_t n) {
     return std::max(al((int64_t)radix_scratch_bytes(n)), bsort::fits(n) ? bsort::work_bytes(n) : 0) +
@@ -834,6 +835,7 @@ struct Epoch {
 
   int run(const hm_tree *t, const int64_t *keys, const int64_t *vals, int flags, bool del, bsort::Ctl *h,
           cudaStream_t s) {
+    if (!slot.ok()) return HM_ENOMEM;
     h->skew = 1;
     if (bsort::fits(n)) {
       bucket_sort(t, keys, s);
@@ -851,7 +853,7 @@ struct Epoch {
 
   int read(bsort::Ctl *h, cudaStream_t s) const {
     const cudaError_t e = cudaGetLastError();
-    return e != cudaSuccess ? cuda_err(e) : read_back(h, ctl, sizeof(*h), s);
+    return e != cudaSuccess ? cuda_err(e) : slot.read(h, ctl, sizeof(*h), s);
   }
 };
 
