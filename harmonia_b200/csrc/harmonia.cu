@@ -472,12 +472,14 @@ void fill_defaults(hm_config *c) {
 // ones take at most 16 KiB: eight CTAs share an SM, and what they stage is taken
 // from its L1, whose hits on the levels below are worth more.  2^20 queries,
 // levels of 19 to 48 KiB staged or not: 2^22 keys 76.5 / 45.0 us, 3 M 73.2 / 44.1,
-// 5 M at fanout 128 78.3 / 51.5; below 16 KiB both the same.  A larger budget is
-// taken at its word.
+// 5 M at fanout 128 78.3 / 51.5; below 16 KiB both the same.  A larger budget,
+// and any other than the default that was set on the loaded tree, is taken at
+// its word.
 constexpr int kSmemDefault = 48 * 1024, kSmemPays = 16 * 1024;
 
 void choose_smem_levels(hm_tree *t) {
-  const int budget = t->cfg.smem_bytes > kSmemDefault ? t->cfg.smem_bytes : std::min(t->cfg.smem_bytes, kSmemPays);
+  const int smem = t->cfg.smem_bytes;
+  const int budget = t->smem_asked || smem > kSmemDefault ? smem : std::min(smem, kSmemPays);
   t->smem_levels = 0;
   t->smem_nodes = 0;
   for (int l = 1; l <= t->height; l++) {
@@ -928,6 +930,7 @@ int hm_set_search_config(hm_tree *t, const hm_config *cfg) {
   if (cfg->join) c.join = cfg->join;
   int rc = check_config(c);
   if (rc) return rc;
+  if (c.smem_bytes != t->cfg.smem_bytes) t->smem_asked = c.smem_bytes != kSmemDefault;
   t->cfg = c;
   t->presort_min = 0;  // an explicit pre-sort applies at every batch size
   choose_smem_levels(t);

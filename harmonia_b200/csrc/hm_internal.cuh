@@ -130,6 +130,7 @@ struct hm_tree {
   int64_t lvl_start[hm::kMaxLevels + 1] = {};
   int smem_levels = 0;
   int smem_nodes = 0;
+  bool smem_asked = false;  // cfg.smem_bytes was set on the loaded tree: taken at its word
   int num_sms = 148;
   int64_t key_min = 0, key_max = 0;  // for the pre-sort digit
   uint64_t generation = 0;           // bumped when the arena is rebuilt

@@ -86,7 +86,7 @@ typedef struct {
                             values load with its keys) */
   int sort_bits;         /* query pre-sort: top bits, 0 = off, 1..16, -1 = auto (default -1) */
   int smem_bytes;        /* budget for top levels staged in shared memory (default 49152;
-                         * up to that, levels are staged while they fit 16384) */
+                            a load with up to that stages levels while they fit 16384) */
   int cache_hints;       /* L2 policy: 1 = inner rows evict_last, leaves evict_first; 2 = none
                             (default 1) */
   int join;              /* large batches: 1 = pre-sort + bucket join, 2 = never, -1 = when the
@@ -220,7 +220,9 @@ int hm_export(hm_tree *t, int64_t *keys, int64_t *vals, size_t cap, size_t *n);
 int hm_tree_get_info(const hm_tree *t, hm_tree_info *info);
 
 /* Changes the search parameters of a loaded tree (group_width,
- * queries_per_group, sort_bits, smem_bytes); layout fields are ignored. */
+ * queries_per_group, sort_bits, smem_bytes); layout fields are ignored.
+ * A smem_bytes other than the present one is taken at its word, unless it is
+ * the default: that one stages what a load does. */
 int hm_set_search_config(hm_tree *t, const hm_config *cfg);
 int hm_get_config(const hm_tree *t, hm_config *cfg);
 
