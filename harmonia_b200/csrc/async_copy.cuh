@@ -54,10 +54,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
   return false;
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 // 2-D tiled TMA load of one box of the tensor map at tmap (the address of a
 // __grid_constant__ kernel parameter) at element coordinates (x, y) into
 // shared memory at address dst; completion is counted on bar.  No multicast.  x times the
@@ -77,8 +73,19 @@ __device__ __forceinline__ void cp_async_element(T *dst, const T *src) {
   static_assert(sizeof(T) == 4 || sizeof(T) == 8, "4 or 8 bytes");
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(sizeof(T)) : "memory");
 }
+// 16 bytes, not kept in L1.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Waits for all but the newest N groups.
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  cp_async_commit();
+  cp_async_wait_group<0>();
 }
 
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }

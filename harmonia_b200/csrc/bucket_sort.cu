@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(kStartThreads) starts_kernel(const uint32_t *_
 constexpr int kScThreads = 256;
 constexpr int kScPer = 8;
 constexpr int kScTile = kScThreads * kScPer;  // pairs of a tile
+static_assert(kScThreads == 256, "a thread per digit");
 
 template <typename V>
 constexpr int scatter_smem() {
@@ -187,33 +188,29 @@ __global__ void __launch_bounds__(kScThreads, 6) scatter_kernel(const int64_t *_
   const Map map = ctl->map;
   int64_t i0, i1;
   uint32_t bucket = 0;
-  if (tid < 256) cnt[tid] = 0;
+  cnt[tid] = 0;
   if constexpr (SECOND) {
     // tiles of first-pass bucket tid: scan, and the bucket this CTA's tile is in
     uint32_t s = 0, e = 0, tiles = 0, incl = 0;
-    if (tid < 256) {
-      if (tid < 1 << l1) {
-        s = start[(uint32_t)tid << l2];
-        e = start[(uint32_t)(tid + 1) << l2];
-        tiles = (e - s + kScTile - 1) / kScTile;
-      }
-      incl = tiles;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      if (lane == 31) wsum[warp] = incl;
+    if (tid < 1 << l1) {
+      s = start[(uint32_t)tid << l2];
+      e = start[(uint32_t)(tid + 1) << l2];
+      tiles = (e - s + kScTile - 1) / kScTile;
     }
+    incl = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
     if (tid == 0) t_end = 0;
     __syncthreads();
-    if (tid < 256) {
-      for (int w = 0; w < warp; w++) incl += wsum[w];
-      if (blockIdx.x < incl && blockIdx.x >= incl - tiles) {
-        t_first = s + (blockIdx.x - (incl - tiles)) * kScTile;
-        t_end = min(e, t_first + kScTile);
-        t_bucket = tid;
-      }
+    for (int w = 0; w < warp; w++) incl += wsum[w];
+    if (blockIdx.x < incl && blockIdx.x >= incl - tiles) {
+      t_first = s + (blockIdx.x - (incl - tiles)) * kScTile;
+      t_end = min(e, t_first + kScTile);
+      t_bucket = tid;
     }
     __syncthreads();
     if (t_end == 0) return;  // past the last tile
@@ -245,24 +242,20 @@ __global__ void __launch_bounds__(kScThreads, 6) scatter_kernel(const int64_t *_
   }
   __syncthreads();
   uint32_t mine = 0, incl = 0, at = 0;
-  if (tid < 256) {
-    mine = cnt[tid];
-    if (mine) at = atomicAdd(cur + bucket + tid, mine);
-    incl = mine;
+  mine = cnt[tid];
+  if (mine) at = atomicAdd(cur + bucket + tid, mine);
+  incl = mine;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane == 31) wsum[warp] = incl;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
   }
+  if (lane == 31) wsum[warp] = incl;
   __syncthreads();
-  if (tid < 256) {
-    uint32_t before = incl - mine;
-    for (int w = 0; w < warp; w++) before += wsum[w];
-    tstart[tid] = before;
-    adj[tid] = at - before;  // slot s of digit d goes to adj[d] + s (modulo 2^32)
-  }
+  uint32_t before = incl - mine;
+  for (int w = 0; w < warp; w++) before += wsum[w];
+  tstart[tid] = before;
+  adj[tid] = at - before;  // slot s of digit d goes to adj[d] + s (modulo 2^32)
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < kScPer; j++) {

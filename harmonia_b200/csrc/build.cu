@@ -33,13 +33,6 @@ __global__ void transform_in_kernel(const int64_t *__restrict__ keys, uint64_t *
     u[i] = (uint64_t)keys[i] ^ kSign;
 }
 
-__global__ void transform_out_kernel(const uint64_t *__restrict__ u, int64_t *__restrict__ keys,
-                                     int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    keys[i] = (int64_t)(u[i] ^ kSign);
-}
-
 // flags bit0: duplicate key, bit1: key == Max_Key.
 __global__ void check_sorted_kernel(const uint64_t *__restrict__ u, int64_t n, unsigned *flags) {
   unsigned f = 0;
@@ -216,12 +209,6 @@ int shape(int64_t n, const hm_config &c, int *height, int64_t *lvl_start, int64_
 void transform_keys_in(const int64_t *keys, uint64_t *ukeys, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
   transform_in_kernel<<<min(blocks_for(n), 148u * 16), kThreads, 0, s>>>(keys, ukeys, n);
-  note_launch();
-}
-
-void transform_keys_out(const uint64_t *ukeys, int64_t *keys, int64_t n, cudaStream_t s) {
-  if (n <= 0) return;
-  transform_out_kernel<<<min(blocks_for(n), 148u * 16), kThreads, 0, s>>>(ukeys, keys, n);
   note_launch();
 }
 

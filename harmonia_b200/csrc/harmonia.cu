@@ -1097,10 +1097,6 @@ int hm_export(hm_tree *t, int64_t *keys, int64_t *vals, size_t cap, size_t *n) {
 
 }  // extern "C"
 
-namespace {
-
-}  // namespace
-
 // The first half of a range scan: where each query's records lie and where
 // they go, until the caller has a place for them.
 struct hm_range_scan {

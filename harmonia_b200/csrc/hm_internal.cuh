@@ -310,7 +310,6 @@ int build_from_pairs(const BuildTarget &b, const int64_t *keys, const int64_t *v
                      int64_t *v1, int64_t *k2, int64_t *v2, void *work, int sms, bsort::Ctl **ctl, cudaStream_t s);
 void check_sorted_keys(const uint64_t *ukeys, int64_t n, unsigned *d_flags, cudaStream_t s);
 void transform_keys_in(const int64_t *keys, uint64_t *ukeys, int64_t n, cudaStream_t s);
-void transform_keys_out(const uint64_t *ukeys, int64_t *keys, int64_t n, cudaStream_t s);
 
 // ---- search (search.cu) ----
 struct SearchLaunch {
@@ -401,7 +400,6 @@ void exclusive_scan_i32(const int32_t *in, int64_t *out, int64_t n, void *scratc
 // leaf_base = exclusive scan of leaf_cnt, unless *go (device memory) is 0.
 void rescan_leaf_base(const hm_tree *t, const unsigned long long *go, void *scratch, cudaStream_t s);
 void export_contents(const hm_tree *t, int64_t *d_keys, int64_t *d_vals, cudaStream_t s);
-size_t range_scratch_bytes(int64_t n);
 // Counts per query: the first len[i] records >= start[i] (end == nullptr), or
 // every record in [start[i], end[i]] (len unused).
 int range_locate(const hm_tree *t, const int64_t *start, const int32_t *len, const int64_t *end, int64_t n,

@@ -88,19 +88,6 @@ __global__ void bucket_bounds_kernel(DevTree t, int f, int64_t lo, int shift, in
   if (b <= nb) leafb[b] = b == 0 ? 0 : past ? t.n_leaf - 1 : leaf;
 }
 
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
 // Words of one leaf in a stage: its keys at a stride of LC + 1 (leaf m's key s
 // at m * (LC + 1) + s, so lanes reading different leaves fall in different
 // banks), then, after all keys, its values densely (m * LC + s).
@@ -132,8 +119,8 @@ __device__ __forceinline__ void stage_leaves(const DevTree &t, const Item &it, S
     const int m = v / (ROW / 2), w = 2 * (v - m * (ROW / 2));
     if (w < LI) continue;
     if (w < LI + LC) {
-      cp_async8(st.kp + m * KS + (w - LI), reinterpret_cast<const int64_t *>(src + v));
-      cp_async8(st.kp + m * KS + (w - LI) + 1, reinterpret_cast<const int64_t *>(src + v) + 1);
+      cp_async_element(st.kp + m * KS + (w - LI), reinterpret_cast<const int64_t *>(src + v));
+      cp_async_element(st.kp + m * KS + (w - LI) + 1, reinterpret_cast<const int64_t *>(src + v) + 1);
     } else {
       cp_async16(st.vp + m * LC + (w - LI - LC), src + v);
     }
@@ -319,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, HM_JOIN_MINB) join_kernel(DevTree t,
     stage_leaves<LC>(t, d[kStages - 1], Stage<LC>(smem + fill * stage_words, ml), ml);
     cp_async_commit();
     const Item dn = it + kStages * g < n_items ? items[it + kStages * g] : none;
-    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");  // the current item's group is done
+    cp_async_wait_group<kStages - 1>();  // the current item's group is done
     __syncthreads();
     const Item cur = d[0];
     const Stage<LC> st(smem + cur_stage * stage_words, ml);
@@ -338,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, HM_JOIN_MINB) join_kernel(DevTree t,
     d[kStages - 1] = dn;
     cur_stage = cur_stage == kStages - 1 ? 0 : cur_stage + 1;
   }
-  cp_async_wait_all();
+  cp_async_wait_group<0>();
 }
 
 // The join for 16-key leaf records: a producer warp fills a ring of stages, the
@@ -361,8 +348,14 @@ __global__ void __launch_bounds__(kThreads, HM_JOIN_MINB) join_kernel(DevTree t,
 // back.  Leaves and queries past the bucket take the last image, so the step
 // back decides between them too: a replayed plan keeps the buckets of its
 // capture, while write epochs may since have put larger keys into the last
-// leaves.  kJoinStep covers a bucket of 256 queries and four standard deviations.  An item takes one CTA barrier: past it every thread
-// has left the item before, whose stage is then filled again.
+// leaves.  An item has kJoinStep queries at most (a bucket of 256 and four
+// standard deviations), so its lookups take one step.  A bucket of more, up to
+// the 767 from which the directory is used, makes two or three items, each of
+// which stages the bucket's leaves; such batches as a whole, against the
+// former items of a whole bucket with one query a thread: 2^24 queries on 2^24
+// keys 516 / 647 us, 2^25 on 2^26 keys 1058 / 1257.  An item takes one CTA
+// barrier: past it every thread has left the item before, whose stage is then
+// filled again.
 // 2^24 queries on 2^26 keys (1.41 GB of records, queries, places and results):
 // 241 us, 5.9 TB/s, 0.90 of the measured copy rate.  Before, with one thread
 // issuing the loads between its lookups, 64-bit binary searches and one query
@@ -448,7 +441,7 @@ __global__ void __launch_bounds__(kJoinThreads + 32, kJoinCtas) join_tma_kernel(
     itm.len_nl = __shfl_sync(0xffffffffu, mine.len_nl, fetched & 31);
     fetched++;
     const int boxes = itm.nl() >= 1 && itm.nl() <= ml ? 2 * ((itm.nl() + 7) >> 3) : 0;
-    const int len = min(itm.len(), kJoinStep);
+    const int len = itm.len();  // kJoinStep at most
     // whole 16-byte words around the queries and the places (both buffers end on 256 bytes)
     const uint32_t qb = len ? ((uint32_t)(len + (itm.qa & 1) + 1) & ~1u) * 8 : 0;
     const uint32_t pb = PLACED && len ? ((uint32_t)(len + (itm.qa & 3) + 3) & ~3u) * 4 : 0;
@@ -509,75 +502,72 @@ __global__ void __launch_bounds__(kJoinThreads + 32, kJoinCtas) join_tma_kernel(
       continue;
     }
     const int len = cur.len();
-    for (int x0 = tid; x0 < len; x0 += kJoinStep) {
-      int64_t q[kJoinQueries], v[kJoinQueries];
-      int32_t qo[kJoinQueries];
-      const bool head = x0 < kJoinStep;  // a fuller bucket's further queries are loaded here
+    if (tid >= len) continue;
+    int64_t q[kJoinQueries], v[kJoinQueries];
+    int32_t qo[kJoinQueries];
+#pragma unroll
+    for (int j = 0; j < kJoinQueries; j++) {
+      const int y = tid + j * kJoinThreads;
+      q[j] = kMaxKey;
+      qo[j] = -1;
+      if (y < len) {
+        qo[j] = cur.qa + y;
+        q[j] = lds64(r + ((cur.qa & 1) + y) * 8);
+        if constexpr (PLACED) qo[j] = (int32_t)lds32(r + kQueryBytes + ((cur.qa & 3) + y) * 4);
+      }
+    }
+    if (staged) {
+      uint32_t qi[kJoinQueries], m4[kJoinQueries];  // 4 * leaf: the last of [1, nl) whose image is <= the key's, else 0
 #pragma unroll
       for (int j = 0; j < kJoinQueries; j++) {
-        const int y = x0 + j * kJoinThreads;
-        q[j] = kMaxKey;
-        qo[j] = -1;
-        if (y < len) {
-          qo[j] = cur.qa + y;
-          q[j] = head ? lds64(r + ((cur.qa & 1) + y) * 8) : __ldg(qs + qo[j]);
-          if constexpr (PLACED)
-            qo[j] = head ? (int32_t)lds32(r + kQueryBytes + ((cur.qa & 3) + y) * 4) : __ldg(place + qo[j]);
-        }
+        const uint64_t qu = biased(q[j]);
+        const uint64_t d = qu <= lo_u ? 0 : (qu - lo_u) >> ishift;
+        qi[j] = d > kImageMax ? kImageMax : (uint32_t)d;
+        m4[j] = 0;
       }
-      if (staged) {
-        uint32_t qi[kJoinQueries], m4[kJoinQueries];  // 4 * leaf: the last of [1, nl) whose image is <= the key's, else 0
 #pragma unroll
-        for (int j = 0; j < kJoinQueries; j++) {
-          const uint64_t qu = biased(q[j]);
-          const uint64_t d = qu <= lo_u ? 0 : (qu - lo_u) >> ishift;
-          qi[j] = d > kImageMax ? kImageMax : (uint32_t)d;
-          m4[j] = 0;
-        }
+      for (uint32_t step = 2 * SPAN; step >= 4; step >>= 1) {
 #pragma unroll
-        for (uint32_t step = 2 * SPAN; step >= 4; step >>= 1) {
+        for (int j = 0; j < kJoinQueries; j++)
+          if (lds32(im + m4[j] + step) <= qi[j]) m4[j] += step;
+      }
+      uint32_t row[kJoinQueries], x[kJoinQueries], c[kJoinQueries];  // c: 8 * slot
+      int64_t key[kJoinQueries];
 #pragma unroll
-          for (int j = 0; j < kJoinQueries; j++)
-            if (lds32(im + m4[j] + step) <= qi[j]) m4[j] += step;
-        }
-        uint32_t row[kJoinQueries], x[kJoinQueries], c[kJoinQueries];  // c: 8 * slot
-        int64_t key[kJoinQueries];
+      for (int j = 0; j < kJoinQueries; j++) {
+        row[j] = kb + (m4[j] << 5);
+        x[j] = (m4[j] << 2) & 0x70u;
+        c[j] = 0;
+      }
+      // the last key <= q of the leaf (Max_Key pads the tail), else slot 0
 #pragma unroll
-        for (int j = 0; j < kJoinQueries; j++) {
-          row[j] = kb + (m4[j] << 5);
-          x[j] = (m4[j] << 2) & 0x70u;
+      for (uint32_t step = LC * 4; step >= 8; step >>= 1) {
+#pragma unroll
+        for (int j = 0; j < kJoinQueries; j++)
+          if (lds64(row[j] + ((c[j] + step) ^ x[j])) <= q[j]) c[j] += step;
+      }
+#pragma unroll
+      for (int j = 0; j < kJoinQueries; j++) key[j] = lds64(row[j] + (c[j] ^ x[j]));
+#pragma unroll
+      for (int j = 0; j < kJoinQueries; j++) {
+        while (key[j] > q[j] && row[j] != kb) {  // the image of this leaf's first key is the key's, but it lies above
+          row[j] -= 128;
+          x[j] = (x[j] - 16) & 0x70u;
           c[j] = 0;
-        }
-        // the last key <= q of the leaf (Max_Key pads the tail), else slot 0
-#pragma unroll
-        for (uint32_t step = LC * 4; step >= 8; step >>= 1) {
-#pragma unroll
-          for (int j = 0; j < kJoinQueries; j++)
+          for (uint32_t step = LC * 4; step >= 8; step >>= 1)
             if (lds64(row[j] + ((c[j] + step) ^ x[j])) <= q[j]) c[j] += step;
+          key[j] = lds64(row[j] + (c[j] ^ x[j]));
         }
-#pragma unroll
-        for (int j = 0; j < kJoinQueries; j++) key[j] = lds64(row[j] + (c[j] ^ x[j]));
-#pragma unroll
-        for (int j = 0; j < kJoinQueries; j++) {
-          while (key[j] > q[j] && row[j] != kb) {  // the image of this leaf's first key is the key's, but it lies above
-            row[j] -= 128;
-            x[j] = (x[j] - 16) & 0x70u;
-            c[j] = 0;
-            for (uint32_t step = LC * 4; step >= 8; step >>= 1)
-              if (lds64(row[j] + ((c[j] + step) ^ x[j])) <= q[j]) c[j] += step;
-            key[j] = lds64(row[j] + (c[j] ^ x[j]));
-          }
-          v[j] = HM_NOT_FOUND;
-          if (key[j] == q[j] && q[j] != kMaxKey) v[j] = lds64(row[j] + block + (c[j] ^ x[j]));
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < kJoinQueries; j++) v[j] = q[j] != kMaxKey ? lookup_scalar<LC>(t, f, q[j]) : HM_NOT_FOUND;
+        v[j] = HM_NOT_FOUND;
+        if (key[j] == q[j] && q[j] != kMaxKey) v[j] = lds64(row[j] + block + (c[j] ^ x[j]));
       }
+    } else {
 #pragma unroll
-      for (int j = 0; j < kJoinQueries; j++)
-        if (qo[j] >= 0) out[qo[j]] = v[j];
+      for (int j = 0; j < kJoinQueries; j++) v[j] = q[j] != kMaxKey ? lookup_scalar<LC>(t, f, q[j]) : HM_NOT_FOUND;
     }
+#pragma unroll
+    for (int j = 0; j < kJoinQueries; j++)
+      if (qo[j] >= 0) out[qo[j]] = v[j];
   }
   // the stages filled past the last item hold arrivals only
 }

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kCopyWarps * 32) range_copy_kernel(
         cp_async_element(vb + x, src + LC);
       }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    cp_async_commit();
     return max(lim - skip, 0);
   };
   // Writes c words at src (16-B aligned like dst - odd) to dst.
@@ -330,9 +330,9 @@ __global__ void __launch_bounds__(kCopyWarps * 32) range_copy_kernel(
     int c_n = 0;
     if (more) {
       c_n = fetch(st ^ 1, &to_n);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      cp_async_wait_group<1>();
     } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      cp_async_wait_group<0>();
     }
     __syncwarp();
     write(buf + st * 2 * kBuf, okeys + to, c);
@@ -395,10 +395,6 @@ void export_contents(const hm_tree *t, int64_t *d_keys, int64_t *d_vals, cudaStr
   export_kernel<<<grid_for_items(t->n_leaf * t->cfg.leaf_cap, 148u * 32), kThreads, 0, s>>>(
       t->view(), t->cfg.leaf_cap, t->leaf_index, d_keys, d_vals);
   note_launch();
-}
-
-size_t range_scratch_bytes(int64_t n) {
-  return (size_t)align_up(n * 4, 256) * 2 + (size_t)align_up(n * 8, 256) + scan_scratch_bytes(n) + 256;
 }
 
 int range_locate(const hm_tree *t, const int64_t *start, const int32_t *len, const int64_t *end, int64_t n,
