@@ -1394,8 +1394,8 @@ int hm_autotune(hm_tree *t, const int64_t *sample_q, size_t n_, hm_config *best)
     }
   }
   // The descent settings serve every batch, a pre-sort only batches at least
-  // as large as the sample (it wins there; its fixed cost of about ten
-  // launches loses on small batches); the join, where it won, serves batches
+  // as large as the sample (it wins there; its fixed cost of five to
+  // seven launches and a memset loses on small batches); the join, where it won, serves batches
   // at least as large as the sample (the automatic choice).
   t->presort_min = best_cfg.sort_bits > 0 ? n : 0;
   if (join_ms < best_ms) {

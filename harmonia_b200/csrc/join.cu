@@ -357,10 +357,11 @@ __global__ void __launch_bounds__(kThreads, HM_JOIN_MINB) join_kernel(DevTree t,
 // barrier: past it every thread has left the item before, whose stage is then
 // filled again.
 // 2^24 queries on 2^26 keys (1.41 GB of records, queries, places and results):
-// 241 us, 5.9 TB/s, 0.90 of the measured copy rate.  Before, with one thread
+// 237 us, 5.95 TB/s, 0.91 of the measured copy rate.  Before, with one thread
 // issuing the loads between its lookups, 64-bit binary searches and one query
 // a thread: 320 us; the producer warp took it to 288, two queries a thread and
-// the fixed step count to 241 (one query a thread: 252).
+// the fixed step count to 241 (one query a thread: 252), one step per item
+// without a loop over steps to 237.
 //
 // Every wait is bounded: on a timeout the CTA records HM_ETIMEOUT in err, waits
 // (bounded) for the loads it issued and returns.

@@ -8,8 +8,8 @@
 // Here a query asks for the first len[i] records with key >= start[i], or
 // (inclusive form) every record with start[i] <= key <= end[i]; a locate pass
 // descends and computes each query's count, an exclusive scan
-// turns counts into offsets, and a copy pass (one warp per query) writes the
-// records contiguously: leaves are ordered, so the records of a query are the
+// turns counts into offsets, and a copy pass (a warp takes up to four queries)
+// writes the records contiguously: leaves are ordered, so the records of a query are the
 // key-ordered run that starts at (leaf, slot) and continues in leaf+1, ...
 #include "ntg.cuh"
 

@@ -84,11 +84,12 @@ __device__ __forceinline__ int match_slot(const int64_t *p, int64_t q, int sub, 
 // 2^26 keys: 18.2 Gq/s at one query per group against 15.4 for the best
 // setting without it; at two queries per group the extra registers cost more
 // than the round trip saves (12.6), so only Q = 1 uses it.
-// What bounds a batch of many tiles is the L1 data pipe (87 % of its peak rate
-// of wavefronts, L2 37 %, DRAM 43 % for 2^20 queries of 2^24 keys): a wavefront
-// per line that a request touches.  With 32 bytes a lane one request covers a
-// group's 128-B line, half as many wavefronts at the leaf (2^20 queries: 60.6 ->
-// 55.6 us at 2^24 keys, 70.7 -> 66.0 at 2^26).  Wider groups would leave lanes idle.
+// What bounds a batch of many tiles is the L1 data pipe: a wavefront per line
+// that a request touches.  With 16 bytes a lane it ran at 87 % of its peak rate
+// (14.9 M wavefronts for 2^20 queries of 2^24 keys; L2 37 %, DRAM 43 %).  With 32
+// bytes a lane one request covers a group's 128-B line, half as many wavefronts
+// at the leaf (12.9 M, 82 % of the peak rate; 2^20 queries: 60.6 -> 55.6 us at
+// 2^24 keys, 70.7 -> 66.0 at 2^26).  Wider groups would leave lanes idle.
 #ifndef HM_LEAF_VALUES_WITH_KEYS
 #define HM_LEAF_VALUES_WITH_KEYS 1
 #endif
