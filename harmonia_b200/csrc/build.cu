@@ -151,15 +151,12 @@ __global__ void __launch_bounds__(bsort::kSortThreads, 5) leaf_sort_kernel(
 
 // One thread per (node, word) of one inner level.  m = nodes of the level
 // below, whose subtree minima are in submin_below; child_base = BFS id of the
-// level below's first node (n_inner for leaves).  Nothing where *skip is set
-// (skip may be null): the leaves were not built then, and the buffers for the
-// minima may hold the inputs of the sort that follows.
+// level below's first node (n_inner for leaves).
 __global__ void inner_kernel(int64_t nodes, int64_t m, int f, int64_t lvl_base,
                              int64_t child_base, const int64_t *__restrict__ submin_below,
                              int64_t *__restrict__ inner, int32_t *__restrict__ prefix,
-                             int64_t *__restrict__ submin_here, const unsigned *skip) {
+                             int64_t *__restrict__ submin_here) {
   pdl_enter();
-  if (skip && *skip) return;
   const int ix = f / 8, row = ix + f;
   const int64_t total = nodes * (int64_t)row;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -219,7 +216,7 @@ void check_sorted_keys(const uint64_t *ukeys, int64_t n, unsigned *d_flags, cuda
   note_launch();
 }
 
-int build_inner(const BuildTarget &b, int64_t *submin, int64_t *tmp, const unsigned *skip, cudaStream_t s);
+int build_inner(const BuildTarget &b, int64_t *submin, int64_t *tmp, cudaStream_t s);
 
 int build_from_sorted(const BuildTarget &b, const uint64_t *ukeys, const int64_t *vals, int64_t n,
                       int64_t *tmp_a, int64_t *tmp_b, cudaStream_t s) {
@@ -229,12 +226,12 @@ int build_from_sorted(const BuildTarget &b, const uint64_t *ukeys, const int64_t
   leaf_kernel<<<min(blocks_for(leaf_words), 148u * 32), kThreads, 0, s>>>(
       ukeys, vals, n, t->n_leaf, lc, t->leaf_index, t->leaf_rows, t->leaf_cnt, t->leaf_base, tmp_a);
   note_launch();
-  return build_inner(b, tmp_a, tmp_b, nullptr, s);
+  return build_inner(b, tmp_a, tmp_b, s);
 }
 
 // The inner levels bottom-up; submin holds each leaf's smallest key, tmp is
-// as large.  *skip != 0 (device memory; skip may be null): nothing is written.
-int build_inner(const BuildTarget &b, int64_t *submin, int64_t *tmp, const unsigned *skip, cudaStream_t s) {
+// as large.
+int build_inner(const BuildTarget &b, int64_t *submin, int64_t *tmp, cudaStream_t s) {
   const BuildTarget *t = &b;
   const int f = t->fanout;
   int64_t *below = submin, *here = tmp;
@@ -243,12 +240,18 @@ int build_inner(const BuildTarget &b, int64_t *submin, int64_t *tmp, const unsig
     int64_t nodes = t->lvl_start[l + 1] - t->lvl_start[l];
     int64_t words = nodes * (int64_t)t->inner_row;
     launch_pdl(inner_kernel, min(blocks_for(words), 148u * 32), kThreads, 0, s, nodes, m, f, t->lvl_start[l],
-               t->lvl_start[l + 1], below, t->inner, t->prefix, here, skip);
+               t->lvl_start[l + 1], below, t->inner, t->prefix, here);
     note_launch();
     std::swap(below, here);
     m = nodes;
   }
   return cuda_err(cudaGetLastError());
+}
+
+size_t build_work_bytes(int64_t n, int64_t n_leaf) {
+  size_t bytes = (size_t)align_up((int64_t)bsort::work_bytes(n), 256);
+  if (bsort::shape_for(n).passes() == 1) bytes += 2 * 8 * (size_t)align_up(n_leaf, 32);
+  return bytes;
 }
 
 int build_from_pairs(const BuildTarget &b, const int64_t *keys, const int64_t *vals, int64_t n, int64_t *k1,
@@ -257,9 +260,16 @@ int build_from_pairs(const BuildTarget &b, const int64_t *keys, const int64_t *v
   *ctl = w.ctl;
   const int passes = bsort::partition_pairs<int64_t>(keys, vals, n, k1, v1, k2, v2, w, sms, s);
   const int64_t *pk = passes == 2 ? k2 : passes == 1 ? k1 : keys, *pv = passes == 2 ? v2 : passes == 1 ? v1 : vals;
-  // the buffers the partition left free hold the subtree minima (after one pass
-  // these may be the inputs, so nothing writes there on skew)
-  int64_t *ta = passes == 1 ? k2 : k1, *tb = passes == 1 ? v2 : v1;
+  // The subtree minima go to the buffers that the partition left free; after one
+  // pass those may be the inputs, which the LSD sort still needs on skew (the
+  // inner levels are then built from nothing, and again after that sort), so the
+  // work area holds them.  A test of skew in inner_kernel instead would add a
+  // load to each level's chain (178 K pairs: 65.2 against 64.3 us).
+  int64_t *ta = k1, *tb = v1;
+  if (passes == 1) {
+    ta = reinterpret_cast<int64_t *>(static_cast<char *>(work) + align_up((int64_t)bsort::work_bytes(n), 256));
+    tb = ta + align_up(b.n_leaf, 32);
+  }
   constexpr int sm = (int)sizeof(bsort::SortSmem<int64_t>);
   opt_in_smem((const void *)leaf_sort_kernel, sm);
   const unsigned grid = 1u << bsort::shape_for(n).bits;
@@ -267,7 +277,7 @@ int build_from_pairs(const BuildTarget &b, const int64_t *keys, const int64_t *v
              static_cast<const uint32_t *>(passes ? w.start : nullptr), (uint32_t)n, (uint32_t)b.n_leaf, b.leaf_cap,
              b.leaf_index, b.leaf_rows, b.leaf_cnt, b.leaf_base, ta, w.ctl);
   note_launch();
-  return build_inner(b, ta, tb, &w.ctl->skew, s);
+  return build_inner(b, ta, tb, s);
 }
 
 }  // namespace hm

@@ -766,7 +766,7 @@ int hm_bulk_load(const int64_t *keys, const int64_t *vals, size_t n_, const hm_c
   size_t tb = align_up(tn * 8, 256);
   const bool bucketed = bsort::fits(n);
   size_t sort_bytes = radix_scratch_bytes(n);
-  if (bucketed) sort_bytes = std::max(sort_bytes, bsort::work_bytes(n));
+  if (bucketed) sort_bytes = std::max(sort_bytes, build_work_bytes(n, t->n_leaf));
   size_t temp_bytes = 4 * tb + align_up((int64_t)sort_bytes, 256) + 256;
   char *temp = nullptr;
   e = dev_alloc(&t->arena, total);

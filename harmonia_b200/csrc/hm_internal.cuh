@@ -300,12 +300,14 @@ int build_from_sorted(const BuildTarget &b, const uint64_t *ukeys, const int64_t
                       int64_t n, int64_t *tmp_a, int64_t *tmp_b, cudaStream_t s);
 // Builds the arrays of b from n pairs in any order (0 < n <= bsort::kMaxPairs)
 // by the bucket sort.  (k1, v1) and (k2, v2) are work buffers of n words (k1
-// and v1 at least n_leaf); keys and vals may be (k2, v2).  Enqueues only; *ctl
+// and v1 at least n_leaf); keys and vals may be (k2, v2); work holds
+// build_work_bytes.  Enqueues only; *ctl
 // receives the device control block that says what came of it (its skew: the
 // keys crowd a bucket, nothing was built and the inputs are untouched).
 namespace bsort {
 struct Ctl;
 }
+size_t build_work_bytes(int64_t n, int64_t n_leaf);
 int build_from_pairs(const BuildTarget &b, const int64_t *keys, const int64_t *vals, int64_t n, int64_t *k1,
                      int64_t *v1, int64_t *k2, int64_t *v2, void *work, int sms, bsort::Ctl **ctl, cudaStream_t s);
 void check_sorted_keys(const uint64_t *ukeys, int64_t n, unsigned *d_flags, cudaStream_t s);
