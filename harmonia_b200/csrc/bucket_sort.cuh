@@ -34,6 +34,10 @@ namespace bsort {
 constexpr int kCap = 2048;     // pairs a bucket may hold: what one CTA sorts
 constexpr int kMean = 1536;    // pairs a bucket averages at most
 constexpr int kMaxBits = 16;   // 2^16 16-bit counters are 128 KiB of shared memory
+// With few buckets the map's whole factor leaves some of them empty (2 of 2.7:
+// 3000 even keys put 2200 into one); with eight the others get an eighth more at
+// most.  3000 even keys load in 44 us, 168 by way of the LSD sort.
+constexpr int kMinBits = 3;
 constexpr int64_t kMaxPairs = (int64_t)kMean << kMaxBits;
 
 // Monotone map of keys to buckets: the offset from lo, shifted up to use all
@@ -91,6 +95,7 @@ inline bool fits(int64_t n) { return n > 0 && n <= kMaxPairs; }
 inline Shape shape_for(int64_t n) {
   Shape s;
   if (n <= kCap) return s;
+  s.bits = kMinBits;
   while (s.bits < kMaxBits && (n >> s.bits) >= kMean) s.bits++;
   s.l2 = s.bits > 8 ? s.bits / 2 : 0;
   s.l1 = s.bits - s.l2;
